@@ -882,6 +882,35 @@ def test_gemm_bf16_tn_on_pairs_of_blocks(M, T, K, out_dtype):
     assert torch.equal(outs[0], outs[1])      # the same k order, the same bits
 
 
+@pytest.mark.parametrize("V", [8191, 8192, 8193, 40001, 151936, 393216, 393220])
+@pytest.mark.parametrize("kind", ["spread", "flat", "equal", "masked", "steep"])
+def test_sampling_nucleus_over_a_cluster_matches_plain(V, kind):
+    """Rows with a nucleus cut at the edges of the vocabularies that a cluster of blocks takes: cuts among few scores, among
+    thousands, among equal ones, with most scores masked, and with shares that keep one score or nearly all."""
+    from vllm_cpp_b200.sampling import Sampler, SamplingOptions
+    rng = np.random.default_rng(V + len(kind))
+    logits = torch.tensor(rng.normal(0, {"spread": 2.5, "flat": 0.05}.get(kind, 1.0), size=(4, V)), dtype=torch.float32)
+    if kind == "equal":
+        logits[:] = 1.5
+        logits[:, V // 3] = 2.0
+    elif kind == "masked":
+        logits[:, torch.tensor(rng.permutation(V)[: V - 50])] = -math.inf
+    elif kind == "steep":
+        logits[:, V - 1] += 60.0
+    opts = [SamplingOptions(0.7, 0.8, 1.1, 4), SamplingOptions(1.3, 0.999, 1.0, 5), SamplingOptions(1.0, 1e-6, 1.0, 6),
+            SamplingOptions(0.9, 0.5, 1.3, 7)]
+    s = Sampler(V, 4, dev())
+    s._need_counts()
+    seen = {0: rng.integers(0, V, 300).tolist() + [V - 1] * 3, 3: [V // 3, V // 3, 0]}
+    for slot, h in seen.items():
+        s.counts[slot] += torch.bincount(torch.tensor(h), minlength=V).to(dev(), torch.int32)
+    got = s.sample(logits.to(dev()), opts, [3, 4, 5, 6], [0, 1, 2, 3]).cpu().tolist()
+    for i, o in enumerate(opts):
+        want = plain_sample(logits[i].numpy(), temperature=o.temperature, top_p=o.top_p, repeat_penalty=o.repeat_penalty,
+                            history=seen.get(i, ()), seed=o.seed, step=3 + i)
+        assert got[i] == want, (i, got[i], want)
+
+
 @pytest.mark.parametrize("I,T,K", [(128, 256, 64), (200, 300, 96), (1536, 2048, 512), (264, 160, 128)])
 def test_gemm_bf16_swiglu_on_pairs_of_blocks(I, T, K):
     from vllm_cpp_b200 import ops

@@ -882,7 +882,8 @@ def sample(logits, params, counts, out, no_nucleus=False):
         _need(counts, "counts", torch.int32)
         assert counts.shape[1] == V
     nb = max(1, min(64, 2 * num_sms() // max(R, 1), V // 2048))
-    if no_nucleus and nb > 1:
+    # (64 rows of 151,936, greedy: 49 us dealt to blocks, 23 in a cluster a row; 16 rows with a temperature: 25 and 33)
+    if no_nucleus and nb > 1 and not (R >= 64 and 8192 <= V <= 393216):
         global launch_count
         from . import workspace
         part_v = workspace.empty((R * nb,), torch.float32, logits.device)
