@@ -131,6 +131,29 @@ def test_sgemm_tn_at_serving_inner_sizes(M, N, K):
     assert torch.equal(out1[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 9, 16, 17, 32, 41, 65])
+@pytest.mark.parametrize("N,K", [(1, 4), (17, 60), (64, 1020), (65, 1024), (100, 2052), (152, 4160)])
+def test_sgemm_tn_sums_in_one_order(M, N, K):
+    """At the edges of the tiles, of the segments of K and of the choice between the kernels: the same sums, bit for bit,
+    from the kernel for few rows, the one for many, and the one for rows that are not 16-byte multiples."""
+    from vllm_cpp_b200 import ops
+    g = torch.Generator(device=dev()).manual_seed(M + K)
+    a, b = torch.randn(M, K, device=dev(), generator=g), torch.randn(N, K, device=dev(), generator=g)
+    out, ragged, single = (torch.full((M, N + 3), 7.0, device=dev()) for _ in range(3))
+    ops.sgemm_tn(a, b, out[:, :N], b_ready=True)
+    want = a.double() @ b.double().T
+    # a chain sums at most 544 products one after the other: sqrt of that many roundings of a running sum of about sqrt(K),
+    # with a factor of 8 for the largest of the results
+    assert (out[:, :N].double() - want).abs().max().item() < 8 * math.sqrt(min(K, 544)) * 2.0 ** -24 * math.sqrt(K)
+    wide = torch.zeros(M, K + 1, device=dev())
+    wide[:, :K] = a
+    ops.sgemm_tn(wide[:, :K], b, ragged[:, :N])
+    for m in range(M):
+        ops.sgemm_tn(a[m:m + 1], b, single[m:m + 1, :N])
+    assert torch.equal(out, ragged) and torch.equal(out, single)
+    assert (out[:, N:] == 7.0).all()
+
+
 def rope_table(hd, theta, n):
     i = torch.arange(hd // 2, dtype=torch.float64)
     ang = torch.arange(n, dtype=torch.float64)[:, None] * theta ** (-2 * i / hd)[None]

@@ -66,7 +66,7 @@ def _declare(L):
         "vcb_gemm_set_pairs": [I],
         "vcb_gemm_bf16_swiglu": [P, P, P, I, I, I, LL, LL, LL, I, I, P, P],
         "vcb_gemm_bf16_qkv": [P, P, I, I, LL, LL, P, P, LL, I, I, P, P, P, I, P, P, I, I, F, I, I, P, P],
-        "vcb_sgemm_tn": [P, P, P, I, I, I, LL, LL, LL, P],
+        "vcb_sgemm_tn": [P, P, P, I, I, I, LL, LL, LL, I, P],
         "vcb_gemm_bf16_plain": [P, P, P, I, I, I, I, LL, LL, LL, P],
         "vcb_attn_paged": [P, P, I, P, LL, P, P, I, P, P, P, P, I, I, P, P, I, I, I, I, I, I, F, P, P],
         "vcb_attn_paged_ex": [P, P, I, P, LL, P, P, I, P, P, P, P, I, I, P, P, I, I, I, I, I, I, F, I, P, P, I, F, P, I, P, I, I, P, I, I, I, P, P],
@@ -403,15 +403,16 @@ def gemm_qkv_rope(w_qkv, x, q_out, pages, slot_map, positions, cos_sin, q_weight
           int(use_norm), float(eps), nh, nkv, _p(status), _stream())
 
 
-def sgemm_tn(a, b, out):
-    """out[M,N] = a[M,K] . b[N,K]^T in true 32-bit."""
+def sgemm_tn(a, b, out, b_ready=False):
+    """out[M,N] = a[M,K] . b[N,K]^T in true 32-bit.  ``b_ready``: no kernel that may still be running writes ``b`` (a
+    weight matrix), so it may be fetched before the kernel ahead in the stream has ended."""
     _need(a, "a", torch.float32, contiguous=False); _need(b, "b", torch.float32, contiguous=False)
     _need(out, "out", torch.float32, contiguous=False)
     M, K = a.shape
     N = b.shape[0]
     assert b.shape[1] == K and out.shape == (M, N)
     assert a.stride(1) == 1 and b.stride(1) == 1 and out.stride(1) == 1
-    _call("vcb_sgemm_tn", _p(a), _p(b), _p(out), M, N, K, a.stride(0), b.stride(0), out.stride(0), _stream())
+    _call("vcb_sgemm_tn", _p(a), _p(b), _p(out), M, N, K, a.stride(0), b.stride(0), out.stride(0), int(b_ready), _stream())
 
 
 def attn_paged(q, out, pages, block_table, q_start, q_len, ctx_len, items, n_items, rows_max, part_o, part_ml,

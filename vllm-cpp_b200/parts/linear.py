@@ -1,7 +1,7 @@
 """Dense projections y = x . W^T with W stored [out, in] as in the checkpoint
 (src/model.cpp:932-944).
 
-float32 engine: the package's FFMA kernel, true 32-bit.  bfloat16 engine: the
+float32 engine: the package's FFMA kernels, true 32-bit.  bfloat16 engine: the
 package's tcgen05/TMA kernel, bfloat16 operands and 32-bit accumulation in TMEM.
 With few tokens the product is a stream of weights from HBM; the inner dimension
 is then cut into slices so that enough blocks are in flight to fill the GPU, each
@@ -79,7 +79,7 @@ def matmul_tn(x: torch.Tensor, w: torch.Tensor, status: torch.Tensor | None = No
         if w.dtype != torch.float32:
             raise ops.KernelError("float32 activations need float32 weights")
         out = workspace.empty((T, N), torch.float32, x.device)
-        ops.sgemm_tn(x, w, out)
+        ops.sgemm_tn(x, w, out, b_ready=True)
         return out
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise ops.KernelError(f"matmul_tn: unsupported operand types {x.dtype} x {w.dtype}")
