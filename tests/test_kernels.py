@@ -958,6 +958,29 @@ def test_gemm_bf16_swiglu_on_pairs_of_blocks(I, T, K):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("tokens", [128, 160, 192, 224])
+@pytest.mark.parametrize("M,T,K,splits", [(256, 1, 64, 1), (300, 161, 200, 1), (520, 223, 1088, 3), (384, 700, 136, 1)])
+def test_gemm_pairs_of_narrower_token_tiles(tokens, M, T, K, splits):
+    """Pairs of blocks with 128 to 224 tokens a unit, at the edges of the tiles: plain, in k-slices, and with the SiLU-gate."""
+    from vllm_cpp_b200 import ops
+    torch.manual_seed(M + T)
+    index = ops.GEMM_PAIR_TOKENS + tokens
+    w = torch.randn(M, K, device=dev(), dtype=torch.bfloat16)
+    x = torch.randn(T, K, device=dev(), dtype=torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device=dev())
+    want = x.double() @ w.double().T
+    S = ops.gemm_effective_splits(K, splits)
+    out = torch.full((S, T, M), 9.0, device=dev()) if S > 1 else torch.full((T, M), 9.0, device=dev())
+    ops.gemm_bf16_tn(w, x, out, S, status, shape=index)
+    # exact products summed in 32-bit: about K * 2^-24 of sums of size sqrt(K), with room for the tensor core's own order
+    torch.testing.assert_close(out.double().sum(0) if S > 1 else out.double(), want, rtol=1e-5, atol=K * 2.0 ** -22)
+    half = torch.empty(T, M // 2, device=dev(), dtype=torch.bfloat16)
+    ops.gemm_bf16_swiglu(w, x, half, status, shape=index)
+    g, u = want[:, 0::2], want[:, 1::2]
+    torch.testing.assert_close(half.double(), g / (1 + torch.exp(-g)) * u, **tol(torch.bfloat16))
+    ops.check_status(status)
+
+
 @pytest.mark.parametrize("M,T,K,splits", [(6144, 256, 4096, 3), (4096, 512, 12288, 4), (1000, 300, 1096, 5), (512, 130, 640, 2)])
 def test_gemm_k_slices_on_pairs_of_blocks(M, T, K, splits):
     """k-slices on the two-block kernel: every slice's 32-bit partial equals the single-block kernel's to the bit

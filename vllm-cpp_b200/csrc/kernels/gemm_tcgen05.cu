@@ -654,9 +654,8 @@ __device__ __forceinline__ void mbar_arrive_block0(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & PEER_BIT_MASK) : "memory");
 }
 
-template <int STAGES>
+template <int BN, int STAGES>
 struct SmemPair {
-    static constexpr int BN = 256;
     static constexpr int A_BYTES = BM * BK * 2;           // one 128-feature tile
     static constexpr int B_BYTES = (BN / 2) * BK * 2;     // this block's half of the token tile
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -667,14 +666,15 @@ struct SmemPair {
     static constexpr int TOTAL = EPI_OFFSET + EPI_BYTES + 1024;
 };
 
-template <int STAGES>
+template <int BN, int STAGES>
 __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_pair_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                          const __grid_constant__ CUtensorMap map_x,
                                                                          GemmArgs g) {
-    using L = SmemPair<STAGES>;
-    constexpr int BN = 256;
-    constexpr uint32_t TMEM_COLS = 512;   // two accumulators of 256 token columns, used in turn
-    constexpr int CHUNK = 64;             // accumulator columns read per wait in the epilogue
+    using L = SmemPair<BN, STAGES>;
+    static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "token columns of a two-block MMA");
+    constexpr uint32_t TMEM_COLS = 512;   // two accumulators of up to 256 token columns, used in turn
+    constexpr uint32_t ACC_COLS = 256;    // from one to the other
+    constexpr int CHUNK = BN % 64 == 0 ? 64 : 32;   // accumulator columns read per wait in the epilogue
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -734,21 +734,35 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_pair_kernel(const __
     if (warp == 0) {
         // ---- TMA producer (in both blocks): its feature tile and its half of the token tile ----
         if (lane == 0) {
+            // a product of one round: the weights of the first ring before the wait for the kernel ahead (no kernel of a step
+            // writes them).  4B sizes, 36 layers of 180 tokens: 4.22 -> 4.11 ms; longer products gain nothing by it.
+            int early = 0;
+            if (units <= pairs) {
+                int m0, n0, kb0, nkb, z;
+                unit_at(pair, m0, n0, kb0, nkb, z);
+                early = min(nkb, STAGES);
+                for (int i = 0; i < early; ++i) {
+                    if (rank == 0) mbar_expect_tx(full_bar(i), 2 * L::STAGE_BYTES);   // both blocks' bytes land on block 0's barrier
+                    tma_load_2d_pair(base + i * L::STAGE_BYTES, &map_w, full_bar(i) & PEER_BIT_MASK, (kb0 + i) * BK, m0 + (int)rank * BM);
+                }
+            }
             pdl_wait();
-            int it = 0, armed = 0;
+            int it = 0, armed = early;
             bool ok = true;
             for (int u = pair; u < units && ok; u += pairs) {
                 int m0, n0, kb0, nkb, z;
                 unit_at(u, m0, n0, kb0, nkb, z);
                 for (int i = 0; i < nkb; ++i, ++it) {
                     const int s = it % STAGES;
-                    if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1u, abort_flag, g.status)) { ok = false; break; }
-                    if (rank == 0) mbar_expect_tx(full_bar(s), 2 * L::STAGE_BYTES);   // both blocks' bytes land on block 0's barrier
                     const uint32_t dst = base + s * L::STAGE_BYTES;
                     const uint32_t bar0 = full_bar(s) & PEER_BIT_MASK;
-                    tma_load_2d_pair(dst, &map_w, bar0, (kb0 + i) * BK, m0 + (int)rank * BM);
+                    if (it >= early) {
+                        if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1u, abort_flag, g.status)) { ok = false; break; }
+                        if (rank == 0) mbar_expect_tx(full_bar(s), 2 * L::STAGE_BYTES);
+                        tma_load_2d_pair(dst, &map_w, bar0, (kb0 + i) * BK, m0 + (int)rank * BM);
+                    }
                     tma_load_2d_pair(dst + L::A_BYTES, &map_x, bar0, (kb0 + i) * BK, n0 + (int)rank * (BN / 2));
-                    armed = it + 1;
+                    armed = max(armed, it + 1);
                 }
             }
             if (*abort_flag && rank == 0) {
@@ -761,7 +775,7 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_pair_kernel(const __
     } else if (warp == 1) {
         // ---- MMA issuer: block 0 only ----
         if (lane == 0 && rank == 0) {
-            // M = 256 (both blocks' lanes), N = 256
+            // M = 256 (both blocks' lanes), N = BN
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
             int it = 0, j = 0;
             bool ok = true;
@@ -781,7 +795,7 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_pair_kernel(const __
                     const uint64_t da = smem_desc(a_addr), db = smem_desc(a_addr + L::A_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        tc_mma_pair(tmem_base + a * BN, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                        tc_mma_pair(tmem_base + a * ACC_COLS, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
                     tc_commit_pair(empty_bar(s));   // frees the stage in both blocks
                 }
                 if (ok) tc_commit_pair(acc_full_bar(a));
@@ -806,7 +820,7 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_pair_kernel(const __
                 uint32_t v[CHUNK / 16][16];
 #pragma unroll
                 for (int b = 0; b < CHUNK / 16; ++b)
-                    tc_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN + c0 + 16 * b), v[b]);
+                    tc_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * ACC_COLS + c0 + 16 * b), v[b]);
                 tc_wait_ld();
                 if (g.qe.q_out != nullptr) {     // uniform over the block: every warp takes part in the barriers
                     float* stage = reinterpret_cast<float*>(gen + L::EPI_OFFSET);
@@ -1002,11 +1016,9 @@ int launch(const void* W, const void* X, const GemmArgs& g, long long ldw, long 
     return launch_maps<BN, STAGES, MT, ACC>(W, g.M, X, g, ldw, ldx, splits, stream);
 }
 
-// Which products of more than 128 tokens without k-slices run on the two-block kernel: 0 none, 1 (the default) those
-// whose 256 x 256 units fill the rounds of the 74 pairs no worse than the single-block kernel's best shape fills
-// those of the 148 SMs -- round for round the pairs measured about 4 % faster (2,048 tokens: qkv 79.4 -> 75.9 us,
-// o 54.4 -> 52.6, gate_up 294 -> 288; 4,096 tokens: 158 -> 147, 106.5 -> 99.9, 600 -> 575, down 330 -> 297) --
-// 2 all of them (tests).  VLLM_CPP_B200_GEMM_PAIRS sets the default.
+// Which products of more than 128 tokens may run on the two-block kernel: 0 none, 1 (the default) those for which
+// choose_shape expects it to be faster, 2 all of them, on units of 256 tokens (tests).  VLLM_CPP_B200_GEMM_PAIRS sets the
+// default.
 int g_pairs = -1;
 int pairs_mode() {
     if (g_pairs < 0) {
@@ -1016,13 +1028,13 @@ int pairs_mode() {
     return g_pairs;
 }
 
-int launch_pair(const void* W, long long w_rows, const void* X, const GemmArgs& g, long long ldw, long long ldx,
-                cudaStream_t stream) {
-    constexpr int STAGES = 6;
-    using L = SmemPair<STAGES>;
+template <int BN, int STAGES>
+int launch_pair_of(const void* W, long long w_rows, const void* X, const GemmArgs& g, long long ldw, long long ldx,
+                   cudaStream_t stream) {
+    using L = SmemPair<BN, STAGES>;
     CUtensorMap mw, mx;
-    if (!tensor_map(W, w_rows, g.K, ldw, BM, &mw) || !tensor_map(X, g.N, g.K, ldx, 128, &mx)) return -3;
-    auto kern = gemm_bf16_tn_pair_kernel<STAGES>;
+    if (!tensor_map(W, w_rows, g.K, ldw, BM, &mw) || !tensor_map(X, g.N, g.K, ldx, BN / 2, &mx)) return -3;
+    auto kern = gemm_bf16_tn_pair_kernel<BN, STAGES>;
     static bool opted = false;
     if (!opted) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
@@ -1033,7 +1045,7 @@ int launch_pair(const void* W, long long w_rows, const void* X, const GemmArgs& 
         opted = true;
     }
     const int unit_rows = 2 * BM;
-    const long long units = (long long)((g.M + unit_rows - 1) / unit_rows) * ((g.N + 255) / 256) * g.splits;
+    const long long units = (long long)((g.M + unit_rows - 1) / unit_rows) * ((g.N + BN - 1) / BN) * g.splits;
     const long long max_pairs = num_sms() / 2;
     const int pairs = (int)(units < max_pairs ? units : max_pairs);
     cudaLaunchConfig_t cfg = {};
@@ -1058,6 +1070,17 @@ int launch_pair(const void* W, long long w_rows, const void* X, const GemmArgs& 
     return 0;
 }
 
+int launch_pair(const void* W, long long w_rows, const void* X, const GemmArgs& g, long long ldw, long long ldx,
+                cudaStream_t stream, int bn = 256) {
+    switch (bn) {
+        case 128: return launch_pair_of<128, 8>(W, w_rows, X, g, ldw, ldx, stream);
+        case 160: return launch_pair_of<160, 7>(W, w_rows, X, g, ldw, ldx, stream);
+        case 192: return launch_pair_of<192, 7>(W, w_rows, X, g, ldw, ldx, stream);
+        case 224: return launch_pair_of<224, 6>(W, w_rows, X, g, ldw, ldx, stream);
+        default: return launch_pair_of<256, 6>(W, w_rows, X, g, ldw, ldx, stream);
+    }
+}
+
 }  // namespace
 
 VCB_TIMELINE_UNIT(gemm)
@@ -1074,7 +1097,8 @@ VCB_API int vcb_gemm_effective_splits(int K, int splits) {
 
 // The unit shapes that are built: tokens per tile (BN), stages of the ring, 128-feature tiles per unit, accumulators.
 enum GemmShape { SHAPE_N16 = 0, SHAPE_N32, SHAPE_N64, SHAPE_N128, SHAPE_N256, SHAPE_M256_N192, SHAPE_M256_N256, SHAPE_PAIR, SHAPE_M256_N160,
-                 SHAPE_COUNT };
+                 SHAPE_COUNT,
+                 SHAPE_PAIR_TOKENS = 1000 };   // + 128, 160, 192 or 224: pairs with that many tokens a unit
 
 namespace {
 int launch_shape(int shape, const void* W, const void* X, const GemmArgs& g, long long ldw, long long ldx, int splits,
@@ -1088,72 +1112,59 @@ int launch_shape(int shape, const void* W, const void* X, const GemmArgs& g, lon
         case SHAPE_M256_N192: return launch<192, 3, 2, 1>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_M256_N160: return launch<160, 3, 2, 1>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_M256_N256: return launch<256, 3, 2, 1>(W, X, g, ldw, ldx, splits, stream);
-        case SHAPE_PAIR:
+        case SHAPE_PAIR: case SHAPE_PAIR_TOKENS + 128: case SHAPE_PAIR_TOKENS + 160: case SHAPE_PAIR_TOKENS + 192: case SHAPE_PAIR_TOKENS + 224:
             if (g.M < 2 * BM) { vcb_set_error("gemm_bf16_tn: pairs of blocks need at least 256 features"); return -1; }
-            return launch_pair(W, g.M, X, g, ldw, ldx, stream);
+            return launch_pair(W, g.M, X, g, ldw, ldx, stream, shape == SHAPE_PAIR ? 256 : shape - SHAPE_PAIR_TOKENS);
     }
     vcb_set_error("gemm_bf16_tn: no unit shape %d (0..%d)", shape, SHAPE_COUNT - 1);
     return -1;
 }
 
-// time of a product on pairs of blocks in the units of pick_shape's costs (token columns a block works through)
-long long pair_cost(int M, int N) {
-    const long long units = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
-    const long long pairs = num_sms() / 2;
-    return ((units + pairs - 1) / pairs) * 256;
-}
+// The unit shapes for more than 128 tokens: what a k-block (64 of K) of a unit takes, plain and beside an epilogue that
+// computes an activation, and what a round of units takes beside its k-blocks, in microseconds.  From 168 products measured
+// with every shape (2,560 to 34,816 features of the 4B, 8B and 14B sizes, 144 to 2,048 tokens).  A k-block hardly depends
+// on a pair's token columns, so narrow units pay by filling a round; beside an activation it gets slower as more of the SMs
+// take part.  The shapes with one accumulator cannot hide their epilogue: 7 us a round, 15 with an activation, which is
+// where they lost most (19,456 features with the SiLU-gate at 640 tokens: 100 us, 70 on pairs of 224).  Taken by this
+// estimate the products are 0.7 % from the best shape on average; by whole rounds of token columns, as before, 5.4 %.
+struct UnitShape { int shape, tiles, tokens, blocks; float k_block, k_block_act, round, round_act; };
+const UnitShape UNIT_SHAPES[] = {
+    {SHAPE_PAIR, 2, 256, 2, 0.375f, 0.414f, 0.5f, 0.5f},
+    {SHAPE_PAIR_TOKENS + 224, 2, 224, 2, 0.370f, 0.410f, 0.5f, 0.5f},
+    {SHAPE_PAIR_TOKENS + 192, 2, 192, 2, 0.366f, 0.406f, 0.5f, 0.5f},
+    {SHAPE_PAIR_TOKENS + 160, 2, 160, 2, 0.360f, 0.400f, 0.5f, 0.5f},
+    {SHAPE_N256, 1, 256, 1, 0.400f, 0.432f, 0.5f, 0.5f},
+    {SHAPE_N128, 1, 128, 1, 0.330f, 0.330f, 0.5f, 0.5f},
+    {SHAPE_M256_N256, 2, 256, 1, 0.730f, 0.800f, 7.f, 15.f},
+    {SHAPE_M256_N192, 2, 192, 1, 0.550f, 0.610f, 7.f, 15.f},
+    {SHAPE_M256_N160, 2, 160, 1, 0.500f, 0.540f, 7.f, 15.f},
+};
 
-int pick_shape(int M, int N, int K, int splits, long long* cost_out = nullptr) {
-    if (cost_out) *cost_out = -1;
+// For M features, N tokens, inner size K.  `act`: the epilogue computes an activation.  `two_acc`: only shapes whose
+// accumulators are drained beside the next unit's products (all whose units are one head or two, too).
+int choose_shape(int M, int N, int K, int splits, bool act, bool two_acc = false) {
     if (N <= 16) return SHAPE_N16;
     if (N <= 32) return SHAPE_N32;
     if (N <= 64) return SHAPE_N64;
     if (N <= 128) return SHAPE_N128;
-    // a sliced product has too few units for the SMs: the smallest units with 256 tokens measured fastest
-    // at every size from 160 to 1,024 tokens
-    if (M <= 128 || splits > 1) return SHAPE_N256;
-    // Units of 128 x 256 (two accumulator buffers: the epilogue of one unit overlaps the MMAs of the next),
-    // 256 x 256 or 256 x 192 tokens: whichever needs the least time over the SMs, counting whole rounds.
-    // Measured at 2,048 tokens the 128 x 256 units are as fast per flop as the 256-feature ones at an inner size
-    // of 4096, so ties go to them; at 12288 the 256 x 256 units, which read the token tile half as often, are
-    // 7 to 9 % faster (down_proj 156 -> 146 us), so there ties go the other way.
-    auto cost = [&](int mt, int bn) {
-        const long long units = (long long)((M + mt * BM - 1) / (mt * BM)) * ((N + bn - 1) / bn);
-        return ((units + num_sms() - 1) / num_sms()) * (long long)(mt * bn);
-    };
-    const long long c1 = cost(1, 256), c2 = cost(2, 256), c3 = cost(2, 192);
-    // 256 x 160 units where they alone fill one round (2,560 features at 2,048 tokens: 130 units for 148 SMs, where
-    // 192-token units make 110 and 256-token units of 128 features make 160, two rounds)
-    const long long c4 = cost(2, 160);
-    // 128 x 128 units draw more from L2 per flop: a k-block of theirs takes 0.29 us where one of 128 x 256 takes 0.36,
-    // four fifths of the time for half the work.  They pay where they fill one round and 256-token units leave a
-    // third of the SMs idle (qkv_proj at 384 tokens: 30.5 -> 24.5 us).
-    const long long c0 = cost(1, 128) * 8 / 5;
-    if (cost_out) *cost_out = std::min(std::min(std::min(c0, c1), std::min(c2, c3)), c4);
-    if (c4 < c0 && c4 < c1 && c4 < c2 && c4 < c3) return SHAPE_M256_N160;
-    if (c0 < c1 && c0 < c2 && c0 < c3) return SHAPE_N128;
-    if (c1 == c2 && c2 <= c3 && K >= 8192) return SHAPE_M256_N256;
-    if (c1 <= c2 && c1 <= c3) return SHAPE_N256;
-    return c3 < c2 ? SHAPE_M256_N192 : SHAPE_M256_N256;
-}
-bool use_pairs(int M, int N, int K, int splits) {
-    const int mode = pairs_mode();
-    if (mode == 0 || N <= 128 || M < 2 * BM) return false;
-    if (mode == 2) return true;
-    if (splits != 1) {
-        // k-slices on pairs: a pair's unit is 256 x 256 where a single block's is 128 x 256, so there are half as many
-        // units for half as many takers; the pairs draw a third less from L2 per k-block.  That pays for the long inner
-        // sizes (down_proj, 12288: 5 to 7 % at 384 to 768 tokens) where the rounds come out no worse, and not for 4096
-        // (qkv_proj at 256 tokens: 18.1 -> 19.7 us).
-        if (K < 8192) return false;
-        const long long pair_units = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) * splits;
-        const long long single_units = (long long)((M + BM - 1) / BM) * ((N + 255) / 256) * splits;
-        const long long pairs = num_sms() / 2;
-        return (pair_units + pairs - 1) / pairs <= (single_units + num_sms() - 1) / num_sms();
+    const bool pairs = pairs_mode() != 0 && M >= 2 * BM;
+    if (pairs && pairs_mode() == 2) return SHAPE_PAIR;
+    if (M <= BM) return SHAPE_N256;
+    const int k_blocks = ((K + BK - 1) / BK + splits - 1) / splits;
+    int best = SHAPE_N256;
+    float best_us = 0.f;
+    for (const UnitShape& c : UNIT_SHAPES) {
+        if (c.blocks == 2 && !pairs) continue;
+        if (c.round > 1.f && (two_acc || splits > 1)) continue;
+        if (c.shape == SHAPE_N128 && splits > 1) continue;     // draws more from L2 per product, and the slices fill the SMs
+        const long long units = (long long)((M + BM * c.tiles - 1) / (BM * c.tiles)) * ((N + c.tokens - 1) / c.tokens) * splits;
+        const long long takers = num_sms() / c.blocks, rounds = (units + takers - 1) / takers;
+        const float fill = (float)units / (float)(rounds * takers);
+        const float k_block = act ? c.k_block_act * (0.6f + 0.46f * fill) : c.k_block;
+        const float us = (float)rounds * ((float)k_blocks * k_block + (act ? c.round_act : c.round));
+        if (best_us == 0.f || us < best_us) { best = c.shape; best_us = us; }
     }
-    long long single = -1;
-    pick_shape(M, N, K, 1, &single);
-    return single > 0 && pair_cost(M, N) * 24 <= single * 25;
+    return best;
 }
 }  // namespace
 
@@ -1173,8 +1184,7 @@ VCB_API int vcb_gemm_bf16_tn_shape(const void* W, const void* X, void* out, int 
     splits = (total_kb + kb_per_split - 1) / kb_per_split;
     GemmArgs g{out, out_dtype, M, N, K, ldc, split_stride, kb_per_split, splits, 0, status};
     if ((flags & VCB_GEMM_AFTER_SMALL_KERNEL) && N <= 16 && vcb_pdl_enabled()) pf_settings(&g.pf_tiles, &g.pf_delay_ns);
-    if (shape < 0 && use_pairs(M, N, K, splits)) return launch_pair(W, M, X, g, ldw, ldx, stream);
-    return launch_shape(shape < 0 ? pick_shape(M, N, K, splits) : shape, W, X, g, ldw, ldx, splits, stream);
+    return launch_shape(shape < 0 ? choose_shape(M, N, K, splits, false) : shape, W, X, g, ldw, ldx, splits, stream);
 }
 
 // out[t][m] = xIELU(W[m] . X[t]), bfloat16, the activation in the epilogue: what bias_act does with the sums of a product
@@ -1189,8 +1199,7 @@ VCB_API int vcb_gemm_bf16_xielu(const void* W, const void* X, void* out, int M, 
     g.act = 6;
     g.act_coef = coef;
     if ((flags & VCB_GEMM_AFTER_SMALL_KERNEL) && N <= 16 && vcb_pdl_enabled()) pf_settings(&g.pf_tiles, &g.pf_delay_ns);
-    if (shape < 0 && use_pairs(M, N, K, 1)) return launch_pair(W, M, X, g, ldw, ldx, stream);
-    return launch_shape(shape < 0 ? pick_shape(M, N, K, 1) : shape, W, X, g, ldw, ldx, 1, stream);
+    return launch_shape(shape < 0 ? choose_shape(M, N, K, 1, true) : shape, W, X, g, ldw, ldx, 1, stream);
 }
 
 // A product over groups of tokens that each meet another matrix (the experts of a routed feed-forward).  W
@@ -1241,8 +1250,7 @@ VCB_API int vcb_gemm_bf16_swiglu(const void* W, const void* X, void* out, int I,
     const int total_kb = (K + BK - 1) / BK;
     GemmArgs g{out, VCB_BF16, 2 * I, N, K, ldc, 0, total_kb, 1, 1, status};
     if ((flags & VCB_GEMM_AFTER_SMALL_KERNEL) && N <= 16 && vcb_pdl_enabled()) pf_settings(&g.pf_tiles, &g.pf_delay_ns);
-    if (shape < 0 && use_pairs(2 * I, N, K, 1)) return launch_pair(W, 2LL * I, X, g, ldw, ldx, stream);
-    return launch_shape(shape < 0 ? pick_shape(2 * I, N, K, 1) : shape, W, X, g, ldw, ldx, 1, stream);
+    return launch_shape(shape < 0 ? choose_shape(2 * I, N, K, 1, true) : shape, W, X, g, ldw, ldx, 1, stream);
 }
 
 // The stacked q, k, v projection of prompt portions with the per-head norm, the rotation and the cache store in its
@@ -1267,12 +1275,8 @@ VCB_API int vcb_gemm_bf16_qkv(const void* W, const void* X, int N, int K, long l
     GemmArgs g{nullptr, VCB_BF16, M, N, K, 0, 0, total_kb, 1, 0, status,
                QkvEpilogue{(__nv_bfloat16*)q_out, (__nv_bfloat16*)pages, page_stride, slot_map, positions, cos_sin, q_gain, k_gain,
                            max_pos, gain_dtype, use_norm, nh, nkv, page_size, num_pages, eps}};
-    // units of one head: 128 features x 256 tokens, or x 128 where those fill the SMs' rounds better (as pick_shape counts)
-    auto rounds = [&](int bn) { return (((long long)(M / BM) * ((N + bn - 1) / bn) + num_sms() - 1) / num_sms()) * bn; };
-    const bool narrow = N <= 128 || rounds(128) * 8 / 5 < rounds(256);
-    // pairs of blocks as for a plain product of these sizes (mode 2, tests: wherever they can run)
-    if ((!narrow || pairs_mode() == 2) && use_pairs(M, N, K, 1)) return launch_pair(W, M, X, g, ldw, ldx, stream);
-    return narrow ? launch<128, 6, 1, 2>(W, X, g, ldw, ldx, 1, stream) : launch<256, 4, 1, 2>(W, X, g, ldw, ldx, 1, stream);
+    // units of one head (two in a pair of blocks); up to 128 tokens the units of 128, whose shared memory has the exchange
+    return launch_shape(N <= 128 ? SHAPE_N128 : choose_shape(M, N, K, 1, false, true), W, X, g, ldw, ldx, 1, stream);
 }
 
 VCB_API int vcb_gemm_bf16_tn(const void* W, const void* X, void* out, int out_dtype, int M, int N, int K,
