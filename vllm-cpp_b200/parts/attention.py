@@ -63,11 +63,9 @@ MAX_CLUSTER_SHARED = 6
 # that lives for one round trip to memory.  Kernel alone, 8B sizes: 256 tokens over 128 keys 47.3 -> 27.4 us (their
 # keys take 20.5 at the copy bandwidth), 128 over 256 36.3 -> 26.2, 64 over 512 28.6 -> 25.6, 256 over 1,024
 # 171 -> 156; with a pair a block or fewer it gains nothing (32 tokens over 2,048 keys: 42.2 against 43.2).
-# Over long contexts the two forms take the same time alone (64 tokens over 4,096 keys: 157 us), but in the step the
-# persistent one is 2 % behind (10.03 -> 10.25 ms): its blocks all end together, so the output projection's blocks are
-# not resident, with their first weights on the way, before the attention is over.  So it is taken where the longest
-# context is known to be at most STREAM_MAX_CONTEXT, and in captured steps, which serve any context of their class,
-# from STREAM_STATIC_PAIRS pairs on, which no pool holds at long contexts.
+# Over long contexts the two forms take the same time alone (64 tokens over 4,096 keys: 157 us).  A step that runs kernel
+# by kernel takes it where its longest context is at most STREAM_MAX_CONTEXT; a captured step, which serves any context of
+# its class, by the number of pairs (STREAM_STATIC_PAIRS is where the kernel alone is sure to gain).
 # Captured steps take it for fewer pairs, too (stream_in_step): over shuffled pages a step of 64 requests gains 13 to 16 %
 # at every context (8B sizes: 500 keys 5.47 -> 4.69 ms, 2,000 8.04 -> 6.81, 4,096 11.41 -> 9.85; 4B, 8,000 keys 16.7 -> 14.3),
 # 100 requests of 30 to 600 keys 6.32 -> 5.43 ms, 33 of 30 to 300 in 64 slots 3.21 -> 2.97; 64 requests spread over 100 to
