@@ -134,6 +134,7 @@ struct GemmArgs {
     int group_rows;
     int act;                  // applied to the sums before they are stored: 0 none, 3 the square of ReLU, 2 SiLU, 6 xIELU
     const float* act_coef;    // xIELU: the factors of its parabola and of its exponential branch
+    int unit_rows, stages;    // units of up to 128 tokens: features a unit (a multiple of 8, at most 128; 0: chosen), stages of the ring
 };
 
 // up x^2 + x/2 above zero, down (e^x - 1 - x) + x/2 below.  (The bracket cancels near zero, to an error of 1e-7 beside the
@@ -155,8 +156,18 @@ struct Smem {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = MT * A_BYTES + B_BYTES;
+    // Up to 128 tokens a unit may have fewer features than a tile has lanes (GemmArgs::unit_rows): its stages are shorter, and
+    // there are as many more of them as fit into the same room.
+    static constexpr bool FLEX = MT == 1 && BN <= 128;
+    static constexpr int MAX_STAGES = FLEX ? 16 : STAGES;
     static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
-    static constexpr int NUM_BARS = 2 * STAGES + 2 * ACC;
+    static constexpr int NUM_BARS = 2 * MAX_STAGES + 2 * ACC;
+    // a stage's 128 rows are read whole by the products, whatever lies beyond the unit's features: the last stage leaves room for that
+    static int stages(int unit_rows) {
+        const int stage = unit_rows * BK * 2 + B_BYTES, beyond = A_BYTES > stage ? A_BYTES - stage : 0;
+        const int n = (BAR_OFFSET - beyond) / stage;
+        return n < MAX_STAGES ? n : MAX_STAGES;
+    }
     // where the q, k, v epilogue passes a head's values between its four warps: 128 features x 32 tokens (rows padded
     // to 33 words), the warps' partial sums of squares, the tokens' factors, positions and slots
     static constexpr int EPI_OFFSET = (BAR_OFFSET + NUM_BARS * 8 + 16 + 15) / 16 * 16;
@@ -380,9 +391,9 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t bars = base + L::BAR_OFFSET;
     auto full_bar = [&](int s) { return bars + 8u * s; };
-    auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
-    auto acc_full_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
-    auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * STAGES + ACC + a); };
+    auto empty_bar = [&](int s) { return bars + 8u * (L::MAX_STAGES + s); };
+    auto acc_full_bar = [&](int a) { return bars + 8u * (2 * L::MAX_STAGES + a); };
+    auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * L::MAX_STAGES + ACC + a); };
     volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(gen + L::BAR_OFFSET + L::NUM_BARS * 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::BAR_OFFSET + L::NUM_BARS * 8 + 8);
 
@@ -390,13 +401,16 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
     tl_mark(VCB_TL_GEMM, 0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_kb = (g.K + BK - 1) / BK;
-    const int unit_rows = BM * MT;   // rows of W per unit
+    const int unit_rows = L::FLEX ? g.unit_rows : BM * MT;   // rows of W per unit
+    const int stages = L::FLEX ? g.stages : STAGES;
+    const int a_bytes = L::FLEX ? unit_rows * BK * 2 : MT * L::A_BYTES;
+    const int stage_bytes = a_bytes + L::B_BYTES;
     const int m_tiles = (g.M + unit_rows - 1) / unit_rows;
     const int n_tiles = (g.N + BN - 1) / BN;
     const int units = m_tiles * n_tiles * g.splits;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
@@ -439,7 +453,8 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
     if (warp == 0) {
         // ---- TMA producer ----
         if (lane == 0) {
-            int it = 0, armed = 0;
+            int it = 0, armed = 0, s = 0;      // k-blocks so far, those on their way, the stage of the next one
+            uint32_t ph = 0;                   // and how often, modulo two, the ring has been round
             bool ok = true;
             // The weights are written by no kernel of the step, so the first ring of weight tiles is requested
             // before waiting for the kernel that produces the activations: the weight stream is already in
@@ -449,10 +464,10 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                 int m0, n0, kb0, nkb, z, mo;
                 if ((int)blockIdx.x < units && g.tile_group == nullptr) {   // (which group a tile has is known only after the wait)
                     unit_at(blockIdx.x, m0, n0, kb0, nkb, z, mo);
-                    early = min(nkb, STAGES);
+                    early = min(nkb, stages);
                     for (int i = 0; i < early; ++i) {
-                        mbar_expect_tx(full_bar(i), L::STAGE_BYTES);
-                        const uint32_t a_dst = base + i * L::STAGE_BYTES;
+                        mbar_expect_tx(full_bar(i), stage_bytes);
+                        const uint32_t a_dst = base + i * stage_bytes;
 #pragma unroll
                         for (int mt = 0; mt < MT; ++mt)
                             tma_load_2d(a_dst + mt * L::A_BYTES, &map_w, full_bar(i), (kb0 + i) * BK,
@@ -485,28 +500,25 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                 int m0, n0, kb0, nkb, z, mo;
                 unit_at(u, m0, n0, kb0, nkb, z, mo);
                 for (int i = 0; i < nkb; ++i, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    const uint32_t a_dst = base + s * L::STAGE_BYTES;
-                    if (it < early) {   // its weight tiles are already on their way
-                        tma_load_2d(a_dst + MT * L::A_BYTES, &map_x, full_bar(s), (kb0 + i) * BK, n0);
-                        continue;
-                    }
-                    if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g.status)) { ok = false; break; }
-                    mbar_expect_tx(full_bar(s), L::STAGE_BYTES);
+                    const uint32_t a_dst = base + s * stage_bytes;
+                    if (it >= early) {   // (the weight tiles of the first ring are already on their way)
+                        if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g.status)) { ok = false; break; }
+                        mbar_expect_tx(full_bar(s), stage_bytes);
 #pragma unroll
-                    for (int mt = 0; mt < MT; ++mt)
-                        tma_load_2d(a_dst + mt * L::A_BYTES, &map_w, full_bar(s), (kb0 + i) * BK,
-                                    mo + m0 + mt * BM);
-                    tma_load_2d(a_dst + MT * L::A_BYTES, &map_x, full_bar(s), (kb0 + i) * BK, n0);
-                    armed = it + 1;
+                        for (int mt = 0; mt < MT; ++mt)
+                            tma_load_2d(a_dst + mt * L::A_BYTES, &map_w, full_bar(s), (kb0 + i) * BK,
+                                        mo + m0 + mt * BM);
+                        armed = it + 1;
+                    }
+                    tma_load_2d(a_dst + a_bytes, &map_x, full_bar(s), (kb0 + i) * BK, n0);
+                    if (++s == stages) { s = 0; ph ^= 1u; }
                 }
             }
             if (*abort_flag) {
                 // let the copies already in flight land before the block goes away
-                for (int i = max(0, armed - STAGES); i < armed; ++i) {
+                for (int i = max(0, armed - stages); i < armed; ++i) {
                     const long long t0 = clock64();
-                    while (!mbar_try(full_bar(i % STAGES), (i / STAGES) & 1) && clock64() - t0 < VCB_WAIT_CLOCKS) {}
+                    while (!mbar_try(full_bar(i % stages), (i / stages) & 1) && clock64() - t0 < VCB_WAIT_CLOCKS) {}
                 }
             }
         }
@@ -514,7 +526,8 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
         // ---- MMA issuer ----
         if (lane == 0) {
             constexpr uint32_t idesc = instr_desc(BN);
-            int it = 0, j = 0;
+            int s = 0, j = 0;
+            uint32_t ph = 0;
             bool ok = true;
             if (g.tile_group != nullptr) pdl_wait();     // (the tiles' groups come from a kernel before this one)
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
@@ -527,13 +540,12 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + a * (MT * ACC_COLS);
-                for (int i = 0; i < nkb; ++i, ++it) {
-                    const int s = it % STAGES;
-                    ok = mbar_wait(full_bar(s), (it / STAGES) & 1, abort_flag, g.status);
+                for (int i = 0; i < nkb; ++i) {
+                    ok = mbar_wait(full_bar(s), ph, abort_flag, g.status);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t a_addr = base + s * L::STAGE_BYTES;
-                    const uint64_t db = smem_desc(a_addr + MT * L::A_BYTES);
+                    const uint32_t a_addr = base + s * stage_bytes;
+                    const uint64_t db = smem_desc(a_addr + a_bytes);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
                         // 16 k = 32 bytes further along the 128-byte rows: +2 in the descriptor's 16-byte units
@@ -543,6 +555,7 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                                    (i > 0 || k > 0) ? 1u : 0u);
                     }
                     tc_commit(empty_bar(s));   // arrives when these MMAs have read the stage
+                    if (++s == stages) { s = 0; ph ^= 1u; }
                 }
                 if (ok) tc_commit(acc_full_bar(a));
             }
@@ -563,10 +576,11 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
             tc_fence_after();
             const uint32_t tmem_d = tmem_base + a * (MT * ACC_COLS);
             const size_t zoff = (size_t)z * g.split_stride;
+            const int m_end = L::FLEX ? min(g.M, m0 + unit_rows) : g.M;     // lanes beyond a unit's features hold what lay behind them in the ring
 #pragma unroll 1
             for (int cc = 0; cc < MT * BN; cc += CHUNK) {
                 const int mt = cc / BN, c0 = cc % BN;
-                if (n0 + c0 >= g.N) continue;   // uniform over the warp
+                if (n0 + c0 >= g.N || (L::FLEX && m0 + q * 32 >= m_end && g.qe.q_out == nullptr)) continue;   // uniform over the warp
                 const int m = m0 + mt * BM + q * 32 + lane;
                 // several TMEM loads in flight before one wait: their latencies overlap
                 uint32_t v[CHUNK / 16][16];
@@ -588,12 +602,12 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                     }
                 }
                 if (g.swiglu) {
-                    swiglu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, g.M, n0 + c0, g.N, lane);
+                    swiglu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, m_end, n0 + c0, g.N, lane);
                 } else if (g.act == 6) {
-                    xielu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, g.M, n0 + c0, g.N, lane, act_up, act_down);
+                    xielu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, m_end, n0 + c0, g.N, lane, act_up, act_down);
                 } else if (g.act == 0 && n0 + c0 + CHUNK <= g.N) {
                     // a whole chunk of tokens, the sums as they are: no branch a column
-                    if (m < g.M) {
+                    if (m < m_end) {
                         if (g.out_dtype == VCB_F32) {
                             float* o = reinterpret_cast<float*>(g.out) + zoff + (size_t)(n0 + c0) * g.ldc + m;
 #pragma unroll
@@ -604,7 +618,7 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                             for (int jj = 0; jj < CHUNK; ++jj) o[(size_t)jj * g.ldc] = __float2bfloat16_rn(__uint_as_float(v[jj / 16][jj % 16]));
                         }
                     }
-                } else if (m < g.M) {
+                } else if (m < m_end) {
                     if (g.out_dtype == VCB_F32) {
                         float* o = reinterpret_cast<float*>(g.out) + zoff;
 #pragma unroll
@@ -1012,12 +1026,34 @@ int num_sms() {
     return n;
 }
 
+// Features a unit of a product of up to 128 tokens: 128, or of 88 to 120 the fewest with which the units still are as many
+// rounds, so that the last round is not left to a few SMs.  Alone on its way a unit takes 0.2 us a k-block, whatever its
+// features: an SM's bytes in flight bound it.  Gate and up of 4,096 inner lanes, 24,576 features: 128 tokens 45.6 us with units of
+// 128, 41.8 of 88 (280 units on 148 SMs) and 55.0 of 80 (a third round), 64 tokens 43.6, 38.5 and 52.3; 19,456 of 2,560, 64
+// tokens 27.3, 24.2 of 88, 25.0 of 72; the head, 151,936 of 2,560, 127.7 and 123.7 of 120.  One round gains nothing by it
+// (4,096 features in four k-slices: 9.2 us with 128 units of 128, 9.4 with 148 of 112).
+int choose_unit_rows(int M, int n_tiles, int splits) {
+    const long long sms = num_sms(), rounds = ((long long)((M + BM - 1) / BM) * splits + sms - 1) / sms;
+    if (n_tiles > 1 || rounds == 1) return BM;
+    for (int rows = 88; rows < BM; rows += 8)
+        if ((long long)((M + rows - 1) / rows) * splits <= rounds * sms) return rows;
+    return BM;
+}
+
 template <int BN, int STAGES, int MT, int ACC>
-int launch_maps(const void* W, long long w_rows, const void* X, const GemmArgs& g, long long ldw, long long ldx, int splits,
+int launch_maps(const void* W, long long w_rows, const void* X, GemmArgs g, long long ldw, long long ldx, int splits,
                 cudaStream_t stream) {
     using L = Smem<BN, STAGES, MT, ACC>;
+    if (!L::FLEX) {
+        g.unit_rows = BM * MT;
+    } else {
+        // (a tile of a grouped product and a head of the q, k, v epilogue are 128 features)
+        if (g.tile_group != nullptr || g.qe.q_out != nullptr) g.unit_rows = BM;
+        else if (g.unit_rows == 0) g.unit_rows = choose_unit_rows(g.M, (g.N + BN - 1) / BN, splits);
+        g.stages = L::stages(g.unit_rows);
+    }
     CUtensorMap mw, mx;
-    if (!tensor_map(W, w_rows, g.K, ldw, BM, &mw) || !tensor_map(X, g.N, g.K, ldx, BN, &mx)) return -3;
+    if (!tensor_map(W, w_rows, g.K, ldw, L::FLEX ? g.unit_rows : BM, &mw) || !tensor_map(X, g.N, g.K, ldx, BN, &mx)) return -3;
     auto kern = gemm_bf16_tn_kernel<BN, STAGES, MT, ACC>;
     static bool opted = false;
     if (!opted) {
@@ -1028,8 +1064,7 @@ int launch_maps(const void* W, long long w_rows, const void* X, const GemmArgs& 
         }
         opted = true;
     }
-    const int unit_rows = BM * MT;
-    const long long units = (long long)((g.M + unit_rows - 1) / unit_rows) * ((g.N + BN - 1) / BN) * splits;
+    const long long units = (long long)((g.M + g.unit_rows - 1) / g.unit_rows) * ((g.N + BN - 1) / BN) * splits;
     const int grid = (int)(units < num_sms() ? units : num_sms());
     launch_pdl(kern, dim3(grid), dim3(NTHREADS), L::TOTAL, stream, mw, mx, g);
     VCB_CHECK_LAUNCH("gemm_bf16_tn");
@@ -1122,11 +1157,16 @@ VCB_API int vcb_gemm_effective_splits(int K, int splits) {
 // The unit shapes that are built: tokens per tile (BN), stages of the ring, 128-feature tiles per unit, accumulators.
 enum GemmShape { SHAPE_N16 = 0, SHAPE_N32, SHAPE_N64, SHAPE_N128, SHAPE_N256, SHAPE_M256_N192, SHAPE_M256_N256, SHAPE_PAIR, SHAPE_M256_N160,
                  SHAPE_COUNT,
-                 SHAPE_PAIR_TOKENS = 1000 };   // + 160, 192 or 224: pairs with that many tokens a unit
+                 SHAPE_PAIR_TOKENS = 1000,     // + 160, 192 or 224: pairs with that many tokens a unit
+                 SHAPE_ROWS = 2000 };          // + 8 to 128 in steps of 8: units of that many features and up to 128 tokens
 
 namespace {
-int launch_shape(int shape, const void* W, const void* X, const GemmArgs& g, long long ldw, long long ldx, int splits,
+int launch_shape(int shape, const void* W, const void* X, GemmArgs g, long long ldw, long long ldx, int splits,
                  cudaStream_t stream) {
+    if (shape > SHAPE_ROWS && shape <= SHAPE_ROWS + BM && shape % 8 == 0) {
+        g.unit_rows = shape - SHAPE_ROWS;
+        shape = g.N <= 16 ? SHAPE_N16 : g.N <= 32 ? SHAPE_N32 : g.N <= 64 ? SHAPE_N64 : SHAPE_N128;
+    }
     switch (shape) {
         case SHAPE_N16: return launch<16, 8, 1, 2>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_N32: return launch<32, 8, 1, 2>(W, X, g, ldw, ldx, splits, stream);
@@ -1327,7 +1367,7 @@ VCB_API int vcb_gemm_bf16_qkv(const void* W, const void* X, int N, int K, long l
                            max_pos, gain_dtype, use_norm, nh, nkv, page_size, num_pages, eps}};
     // units of one head (two in a pair of blocks); up to 128 tokens the units of 128, whose shared memory has the exchange
     if (shape < 0) shape = N <= 128 ? SHAPE_N128 : choose_shape(M, N, K, 1, EPI_HEADS);
-    VCB_CHECK_ARG(shape == SHAPE_N128 || shape == SHAPE_N256 || shape == SHAPE_PAIR || shape > SHAPE_PAIR_TOKENS,
+    VCB_CHECK_ARG(shape == SHAPE_N128 || shape == SHAPE_N256 || shape == SHAPE_PAIR || (shape > SHAPE_PAIR_TOKENS && shape < SHAPE_ROWS),
                   "gemm_bf16_qkv: unit shape %d has no room for the epilogue's exchange", shape);
     return launch_shape(shape, W, X, g, ldw, ldx, 1, stream);
 }

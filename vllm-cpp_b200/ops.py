@@ -317,6 +317,7 @@ def gemm_effective_splits(K: int, splits: int) -> int:
 
 
 GEMM_PAIR_TOKENS = 1000     # + 160, 192 or 224: the unit shape of pairs of blocks with that many tokens
+GEMM_ROWS = 2000            # + 8 to 128 in steps of 8: units of that many features and up to 128 tokens
 GEMM_SHAPES = ("n16", "n32", "n64", "n128", "n256", "m256_n192", "m256_n256", "pair", "m256_n160")   # unit shapes of the kernel, by index
 
 
