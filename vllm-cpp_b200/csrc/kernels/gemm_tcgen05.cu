@@ -229,17 +229,12 @@ __device__ __forceinline__ void swiglu_store(uint32_t (*v)[16], __nv_bfloat16* o
     }
 }
 
-// xIELU of a chunk's sums, bfloat16, two neighbouring features (lanes) a store: of every two tokens the even lane stores
-// the first and the odd lane the second, each with its neighbour's value.
+// A chunk's results, bfloat16, two neighbouring features (lanes) a store: of every two tokens the even lane stores the first
+// and the odd lane the second, each with its neighbour's value.  Every lane of the warp must call it.
 template <int CHUNK>
-__device__ __forceinline__ void xielu_store(const uint32_t (&v)[CHUNK / 16][16], __nv_bfloat16* out, long long ldc, int m, int M, int t0,
-                                            int N, int lane, float up, float down) {
-    // all values first, without a branch, so that their latencies overlap (as in swiglu_store)
-    float r[CHUNK];
-#pragma unroll
-    for (int jj = 0; jj < CHUNK; ++jj) r[jj] = gemm_xielu(__uint_as_float(v[jj / 16][jj % 16]), up, down);
+__device__ __forceinline__ void pair_store(const float (&r)[CHUNK], __nv_bfloat16* out, long long ldc, int m, int M, int t0, int N, int lane) {
     const bool odd = lane & 1;
-    if (((M | (int)ldc) & 1) == 0) {        // uniform
+    if (((M | (int)ldc) & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0) {        // uniform
         __nv_bfloat162 p[CHUNK / 2];
 #pragma unroll
         for (int jj = 0; jj < CHUNK; jj += 2) {
@@ -262,6 +257,44 @@ __device__ __forceinline__ void xielu_store(const uint32_t (&v)[CHUNK / 16][16],
 #pragma unroll
         for (int jj = 0; jj < CHUNK; ++jj)
             if (t0 + jj < N) o[(size_t)jj * ldc] = __float2bfloat16_rn(r[jj]);
+    }
+}
+
+// xIELU of a chunk's sums
+template <int CHUNK>
+__device__ __forceinline__ void xielu_store(const uint32_t (&v)[CHUNK / 16][16], __nv_bfloat16* out, long long ldc, int m, int M, int t0,
+                                            int N, int lane, float up, float down) {
+    // all values first, without a branch, so that their latencies overlap (as in swiglu_store)
+    float r[CHUNK];
+#pragma unroll
+    for (int jj = 0; jj < CHUNK; ++jj) r[jj] = gemm_xielu(__uint_as_float(v[jj / 16][jj % 16]), up, down);
+    pair_store<CHUNK>(r, out, ldc, m, M, t0, N, lane);
+}
+
+// A chunk's sums after an activation (gemm_act), 32-bit or bfloat16.  A last chunk that is not whole stores under a predicate a
+// column, nothing else: with the activation behind each column's branch it took a product 6 to 13 us longer than a whole one.
+template <int CHUNK>
+__device__ __forceinline__ void plain_store(const uint32_t (&v)[CHUNK / 16][16], void* out, int out_dtype, size_t at, long long ldc, int m, int M,
+                                            int t0, int N, int lane, int act) {
+    float r[CHUNK];
+#pragma unroll
+    for (int jj = 0; jj < CHUNK; ++jj) r[jj] = __uint_as_float(v[jj / 16][jj % 16]);
+    if (act != 0) {
+#pragma unroll
+        for (int jj = 0; jj < CHUNK; ++jj) r[jj] = gemm_act(r[jj], act);
+    }
+    if (out_dtype == VCB_BF16) {
+        pair_store<CHUNK>(r, reinterpret_cast<__nv_bfloat16*>(out) + at, ldc, m, M, t0, N, lane);
+    } else if (m < M) {
+        float* o = reinterpret_cast<float*>(out) + at + (size_t)t0 * ldc + m;
+        if (t0 + CHUNK <= N) {
+#pragma unroll
+            for (int jj = 0; jj < CHUNK; ++jj) o[(size_t)jj * ldc] = r[jj];
+        } else {
+#pragma unroll
+            for (int jj = 0; jj < CHUNK; ++jj)
+                if (t0 + jj < N) o[(size_t)jj * ldc] = r[jj];
+        }
     }
 }
 
@@ -605,32 +638,8 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                     swiglu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, m_end, n0 + c0, g.N, lane);
                 } else if (g.act == 6) {
                     xielu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, m_end, n0 + c0, g.N, lane, act_up, act_down);
-                } else if (g.act == 0 && n0 + c0 + CHUNK <= g.N) {
-                    // a whole chunk of tokens, the sums as they are: no branch a column
-                    if (m < m_end) {
-                        if (g.out_dtype == VCB_F32) {
-                            float* o = reinterpret_cast<float*>(g.out) + zoff + (size_t)(n0 + c0) * g.ldc + m;
-#pragma unroll
-                            for (int jj = 0; jj < CHUNK; ++jj) o[(size_t)jj * g.ldc] = __uint_as_float(v[jj / 16][jj % 16]);
-                        } else {
-                            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(g.out) + zoff + (size_t)(n0 + c0) * g.ldc + m;
-#pragma unroll
-                            for (int jj = 0; jj < CHUNK; ++jj) o[(size_t)jj * g.ldc] = __float2bfloat16_rn(__uint_as_float(v[jj / 16][jj % 16]));
-                        }
-                    }
-                } else if (m < m_end) {
-                    if (g.out_dtype == VCB_F32) {
-                        float* o = reinterpret_cast<float*>(g.out) + zoff;
-#pragma unroll
-                        for (int jj = 0; jj < CHUNK; ++jj)
-                            if (n0 + c0 + jj < g.N) o[(size_t)(n0 + c0 + jj) * g.ldc + m] = gemm_act(__uint_as_float(v[jj / 16][jj % 16]), g.act);
-                    } else {
-                        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(g.out) + zoff;
-#pragma unroll
-                        for (int jj = 0; jj < CHUNK; ++jj)
-                            if (n0 + c0 + jj < g.N)
-                                o[(size_t)(n0 + c0 + jj) * g.ldc + m] = __float2bfloat16_rn(gemm_act(__uint_as_float(v[jj / 16][jj % 16]), g.act));
-                    }
+                } else {
+                    plain_store<CHUNK>(v, g.out, g.out_dtype, zoff, g.ldc, m, m_end, n0 + c0, g.N, lane, g.act);
                 }
             }
             tc_fence_before();
@@ -879,32 +888,8 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_pair_kernel(const __
                     swiglu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, g.M, n0 + c0, g.N, lane);
                 } else if (g.act == 6) {
                     xielu_store<CHUNK>(v, reinterpret_cast<__nv_bfloat16*>(g.out), g.ldc, m, g.M, n0 + c0, g.N, lane, act_up, act_down);
-                } else if (g.act == 0 && n0 + c0 + CHUNK <= g.N) {
-                    // a whole chunk of tokens, the sums as they are: no branch a column
-                    if (m < g.M) {
-                        if (g.out_dtype == VCB_F32) {
-                            float* o = reinterpret_cast<float*>(g.out) + zoff + (size_t)(n0 + c0) * g.ldc + m;
-#pragma unroll
-                            for (int jj = 0; jj < CHUNK; ++jj) o[(size_t)jj * g.ldc] = __uint_as_float(v[jj / 16][jj % 16]);
-                        } else {
-                            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(g.out) + zoff + (size_t)(n0 + c0) * g.ldc + m;
-#pragma unroll
-                            for (int jj = 0; jj < CHUNK; ++jj) o[(size_t)jj * g.ldc] = __float2bfloat16_rn(__uint_as_float(v[jj / 16][jj % 16]));
-                        }
-                    }
-                } else if (m < g.M) {
-                    if (g.out_dtype == VCB_F32) {
-                        float* o = reinterpret_cast<float*>(g.out) + zoff;
-#pragma unroll
-                        for (int jj = 0; jj < CHUNK; ++jj)
-                            if (n0 + c0 + jj < g.N) o[(size_t)(n0 + c0 + jj) * g.ldc + m] = gemm_act(__uint_as_float(v[jj / 16][jj % 16]), g.act);
-                    } else {
-                        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(g.out) + zoff;
-#pragma unroll
-                        for (int jj = 0; jj < CHUNK; ++jj)
-                            if (n0 + c0 + jj < g.N)
-                                o[(size_t)(n0 + c0 + jj) * g.ldc + m] = __float2bfloat16_rn(gemm_act(__uint_as_float(v[jj / 16][jj % 16]), g.act));
-                    }
+                } else {
+                    plain_store<CHUNK>(v, g.out, g.out_dtype, zoff, g.ldc, m, g.M, n0 + c0, g.N, lane, g.act);
                 }
             }
             tc_fence_before();
