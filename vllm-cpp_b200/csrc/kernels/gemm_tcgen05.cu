@@ -1174,43 +1174,43 @@ int launch_shape(int shape, const void* W, const void* X, GemmArgs g, long long 
 //   one accumulator:   once + rounds * (k_blocks * k_block * (1 + busy * fill) + drain) + ragged
 // A k-block is 64 of K; fill is the share of a round's units that there are (a k-block gets slower as more of the SMs draw
 // from L2); drain is a unit's epilogue, hidden behind the next unit's products only where there is a second accumulator, and
-// then only if those take longer (short K); ragged is what a last chunk of tokens that is not whole adds, whose columns are
-// stored one by one.  The epilogues differ so much that each kind has numbers of its own.
-// Fitted to every shape at 3,686 sizes a kind (256 to 34,816 features, 129 to 4,096 tokens, K of 128 to 12,288; heads 1,440).
-// Taken by the estimate the products are on average 0.8 % (plain), 1.3 (k-slices), 0.3 (SiLU-gate), 0.3 (xIELU) and 1.0 (heads)
-// from the best shape.  Fitted to K from 2,560 on, with one constant a round and none for ragged tokens, it was 5.1, 3.6, 5.4,
-// 1.9 and 1.4 %, and short inner sizes were up to 1.67 times as slow as by whole rounds of token columns, the rule before that
-// (5,120 gate and up rows of 256 lanes, 911 tokens: 28 us by rounds, 46 then).  By rounds: 6.8, 11.8, 5.1, 2.1 and 4.1 %.
+// then only if those take longer (short K); ragged is what a last chunk of tokens that is not whole adds.  The epilogues differ
+// so much that each kind has numbers of its own.
+// Fitted to every shape, launches one behind the other with weights from HBM: plain and SiLU-gate at 627 and 1,330 sizes (1,024 to
+// 34,816 features, 130 to 4,096 tokens, K of 256 to 9,728), the others at 3,686 (heads 1,440).  Taken by the estimate the products
+// are on average 0.5 % (plain), 0.3 (SiLU-gate), 1.3 (k-slices), 0.3 (xIELU) and 1.0 (heads) from the best shape; by the numbers
+// that fitted the first two epilogues before they shared columns between lanes, 3.9 and 1.3 %, and up to 48 (1,024 features of 256
+// lanes, 911 tokens).  By whole rounds of token columns, the rule before the estimate: 6.8, 5.1, 11.8, 2.1 and 4.1 %.
 enum Epilogue { EPI_PLAIN = 0, EPI_PARTIAL, EPI_GATE, EPI_XIELU, EPI_HEADS, EPI_COUNT };
 struct UnitTime { float k_block, busy, start, drain, once, ragged; };      // k_block 0: not taken
 struct UnitShape { int shape, tiles, tokens, blocks, chunk; UnitTime time[EPI_COUNT]; };
 const UnitShape UNIT_SHAPES[] = {
     {SHAPE_PAIR, 2, 256, 2, 64,
-     {{0.284f, 0.19f, 2.0f, 0.0f, 10.5f, 6.0f}, {0.286f, 0.35f, 2.0f, 0.0f, 10.4f, 6.2f}, {0.283f, 0.17f, 7.4f, 10.5f, 3.3f, 0.0f},
+     {{0.264f, 0.28f, 1.5f, 0.4f, 4.6f, 0.2f}, {0.286f, 0.35f, 2.0f, 0.0f, 10.4f, 6.2f}, {0.276f, 0.28f, 0.9f, 3.3f, 1.6f, 0.1f},
       {0.280f, 0.24f, 2.3f, 4.0f, 7.8f, 0.0f}, {0.254f, 0.16f, 8.6f, 8.6f, 11.4f, 0.0f}}},
     {SHAPE_PAIR_TOKENS + 224, 2, 224, 2, 32,
-     {{0.280f, 0.19f, 1.4f, 3.1f, 7.9f, 0.6f}, {0.281f, 0.29f, 1.4f, 2.3f, 8.7f, 1.0f}, {0.286f, 0.08f, 6.6f, 9.6f, 3.1f, 0.0f},
+     {{0.268f, 0.21f, 1.3f, 3.0f, 1.7f, 0.0f}, {0.281f, 0.29f, 1.4f, 2.3f, 8.7f, 1.0f}, {0.274f, 0.22f, 0.9f, 3.5f, 1.4f, 0.1f},
       {0.277f, 0.20f, 2.5f, 4.2f, 6.8f, 0.0f}, {0.258f, 0.07f, 8.5f, 4.5f, 13.2f, 0.0f}}},
     {SHAPE_PAIR_TOKENS + 192, 2, 192, 2, 64,
-     {{0.291f, 0.09f, 1.3f, 0.0f, 10.6f, 7.3f}, {0.292f, 0.12f, 1.4f, 0.0f, 10.4f, 6.1f}, {0.300f, 0.00f, 5.6f, 8.8f, 4.0f, 0.0f},
+     {{0.268f, 0.16f, 1.0f, 1.9f, 2.9f, 0.4f}, {0.292f, 0.12f, 1.4f, 0.0f, 10.4f, 6.1f}, {0.278f, 0.16f, 0.7f, 2.6f, 2.1f, 0.3f},
       {0.284f, 0.14f, 1.8f, 3.0f, 8.5f, 0.4f}, {0.283f, 0.00f, 6.2f, 9.2f, 8.5f, 0.0f}}},
     {SHAPE_PAIR_TOKENS + 160, 2, 160, 2, 32,
-     {{0.287f, 0.12f, 0.8f, 2.4f, 8.4f, 1.6f}, {0.287f, 0.14f, 0.9f, 1.8f, 9.1f, 1.5f}, {0.300f, 0.00f, 4.3f, 7.6f, 4.6f, 0.0f},
+     {{0.280f, 0.11f, 0.8f, 2.3f, 2.4f, 0.1f}, {0.287f, 0.14f, 0.9f, 1.8f, 9.1f, 1.5f}, {0.282f, 0.11f, 0.6f, 2.7f, 2.0f, 0.2f},
       {0.284f, 0.14f, 1.5f, 3.2f, 7.7f, 0.0f}, {0.274f, 0.00f, 5.5f, 3.1f, 13.7f, 0.0f}}},
     {SHAPE_N256, 1, 256, 1, 64,
-     {{0.356f, 0.08f, 2.2f, 0.0f, 9.0f, 7.5f}, {0.348f, 0.30f, 2.2f, 0.0f, 8.8f, 4.4f}, {0.364f, 0.11f, 4.1f, 8.8f, 3.8f, 0.0f},
+     {{0.309f, 0.26f, 0.9f, 3.0f, 0.8f, 0.1f}, {0.348f, 0.30f, 2.2f, 0.0f, 8.8f, 4.4f}, {0.315f, 0.26f, 0.5f, 3.4f, 0.4f, 0.2f},
       {0.349f, 0.14f, 2.3f, 4.3f, 5.8f, 0.0f}, {0.322f, 0.05f, 8.0f, 7.7f, 10.7f, 0.0f}}},
     {SHAPE_N128, 1, 128, 1, 64,
-     {{0.258f, 0.14f, 0.9f, 1.9f, 6.9f, 5.5f}, {}, {0.268f, 0.06f, 2.4f, 5.6f, 5.1f, 0.0f},
+     {{0.240f, 0.14f, 0.7f, 1.5f, 2.5f, 0.2f}, {}, {0.247f, 0.13f, 0.4f, 2.0f, 1.6f, 0.2f},
       {0.254f, 0.16f, 1.1f, 2.6f, 7.1f, 0.0f}, {0.261f, 0.00f, 3.5f, 6.7f, 7.4f, 0.0f}}},
     {SHAPE_M256_N256, 2, 256, 1, 64,
-     {{0.567f, 0.29f, 0.0f, 5.9f, 8.0f, 13.0f}, {}, {0.557f, 0.37f, 0.0f, 20.5f, 7.6f, 0.0f},
+     {{0.543f, 0.26f, 0.0f, 4.5f, 2.8f, 0.3f}, {}, {0.537f, 0.30f, 0.0f, 5.6f, 2.7f, 0.2f},
       {0.563f, 0.32f, 0.0f, 7.7f, 8.4f, 0.0f}, {}}},
     {SHAPE_M256_N192, 2, 192, 1, 64,
-     {{0.499f, 0.18f, 0.0f, 3.9f, 8.1f, 12.0f}, {}, {0.492f, 0.23f, 0.0f, 15.9f, 7.9f, 0.0f},
+     {{0.453f, 0.24f, 0.0f, 3.2f, 2.8f, 0.6f}, {}, {0.435f, 0.31f, 0.0f, 3.9f, 2.6f, 0.6f},
       {0.493f, 0.21f, 0.0f, 5.8f, 8.6f, 0.9f}, {}}},
     {SHAPE_M256_N160, 2, 160, 1, 32,
-     {{0.457f, 0.19f, 0.0f, 3.6f, 8.4f, 2.1f}, {}, {0.460f, 0.20f, 0.0f, 12.6f, 8.3f, 0.0f},
+     {{0.410f, 0.23f, 0.0f, 3.1f, 2.6f, 0.3f}, {}, {0.390f, 0.33f, 0.0f, 3.9f, 2.6f, 0.3f},
       {0.457f, 0.19f, 0.0f, 5.3f, 8.4f, 0.4f}, {}}},
 };
 
