@@ -130,6 +130,8 @@ __global__ __launch_bounds__(TK) void attn_paged_kernel(AttnArgs a) {
     int* lo_s = reinterpret_cast<int*>(db_s + RMAX);   // [RMAX] first key of the row's window
     long long* voff_s = reinterpret_cast<long long*>(lo_s + RMAX);  // [TK] element offset of each key's V row
 
+    pdl_trigger();
+    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int* item = a.items + (size_t)blockIdx.x * ITEM_INTS;
     const int e = item[0], q0 = item[1], slice = item[3], nslices = item[4], dec_index = item[5];
@@ -465,7 +467,7 @@ int launch_attn(const AttnArgs& a, int n_items, cudaStream_t stream) {
             return -2;
         }
     }
-    kern<<<dim3(n_items, a.nkv * hchunks, zblocks), TK, smem, stream>>>(a);
+    launch_pdl(kern, dim3(n_items, a.nkv * hchunks, zblocks), dim3(TK), smem, stream, a);
     VCB_CHECK_LAUNCH("attn_paged");
     return 0;
 }

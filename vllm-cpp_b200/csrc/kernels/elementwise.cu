@@ -9,6 +9,8 @@
 // SiLU src/model.cpp:964-966, page write src/paged_attention.cpp:127-142.
 #include "common.cuh"
 
+#include <type_traits>
+
 #include <stdarg.h>
 #include <stdlib.h>
 
@@ -74,6 +76,8 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ resid, const void* __rest
     extern __shared__ float smem[];
     float* xs = smem;
     float* scratch = smem + H;
+    pdl_trigger();
+    pdl_wait();
     const int i = blockIdx.x;
     const size_t r = rows ? (size_t)rows[i] : (size_t)i;
     const bool write_back = rows == nullptr && S > 0;
@@ -91,12 +95,26 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ resid, const void* __rest
         store_from_f32(out, out_dtype, (size_t)i * H + h, load_as_f32(w, w_dtype, h) * xs[h] * inv);
 }
 
-// Same contract for the shapes serving uses (H a multiple of 4, 32-bit deltas, bfloat16 out): 16-byte loads, every
-// load of a row issued before any is used, the row kept in registers.  VPT = float4s per thread.
-template <int VPT>
+// four neighbouring numbers in one store
+__device__ __forceinline__ void store4(__nv_bfloat16* out, int c, float x, float y, float z, float w) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(x, y), hi = __floats2bfloat162_rn(z, w);
+    uint2 pk;
+    pk.x = *reinterpret_cast<uint32_t*>(&lo);
+    pk.y = *reinterpret_cast<uint32_t*>(&hi);
+    reinterpret_cast<uint2*>(out)[c] = pk;
+}
+__device__ __forceinline__ void store4(float* out, int c, float x, float y, float z, float w) {
+    reinterpret_cast<float4*>(out)[c] = make_float4(x, y, z, w);
+}
+
+// Same contract for the shapes serving uses (H a multiple of 4, 32-bit deltas): 16-byte loads, every load of a row issued
+// before any is used, the row kept in registers.  VPT = float4s per thread.
+// Bound by its one round trip to memory.  The 32-bit engine's rows come here too: with them, and with its norms and its attention
+// launched before the kernel ahead has ended, a step of three tokens of the 4B sizes went from 4,930 to 4,499 us.
+template <int VPT, typename T>
 __global__ __launch_bounds__(1024) void add_rmsnorm_vec_kernel(float* __restrict__ resid, const float* __restrict__ delta,
                                                                int S, size_t delta_stride, const void* __restrict__ w,
-                                                               int w_dtype, float eps, __nv_bfloat16* __restrict__ out,
+                                                               int w_dtype, float eps, T* __restrict__ out,
                                                                const int* __restrict__ rows, int H) {
     __shared__ float scratch[33];
     pdl_trigger();
@@ -167,14 +185,9 @@ __global__ __launch_bounds__(1024) void add_rmsnorm_vec_kernel(float* __restrict
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
         const int c = threadIdx.x + v * blockDim.x;
-        if (c < H4) {
-            __nv_bfloat162 lo = __floats2bfloat162_rn(gain[v].x * x[v].x * inv, gain[v].y * x[v].y * inv);
-            __nv_bfloat162 hi = __floats2bfloat162_rn(gain[v].z * x[v].z * inv, gain[v].w * x[v].w * inv);
-            uint2 pk;
-            pk.x = *reinterpret_cast<uint32_t*>(&lo);
-            pk.y = *reinterpret_cast<uint32_t*>(&hi);
-            reinterpret_cast<uint2*>(out + (size_t)i * H)[c] = pk;
-        }
+        if (c < H4)
+            store4(out + (size_t)i * H, c, gain[v].x * x[v].x * inv, gain[v].y * x[v].y * inv, gain[v].z * x[v].z * inv,
+                   gain[v].w * x[v].w * inv);
     }
     tl_mark(VCB_TL_NORM, 2);
 }
@@ -232,14 +245,9 @@ __global__ __launch_bounds__(1024) void add_rmsnorm_stream_kernel(float* __restr
 #pragma unroll
         for (int v = 0; v < VPT; ++v) {
             const int c = threadIdx.x + v * blockDim.x;
-            if (c < H4) {
-                __nv_bfloat162 lo = __floats2bfloat162_rn(gain[v].x * xr[v].x * inv, gain[v].y * xr[v].y * inv);
-                __nv_bfloat162 hi = __floats2bfloat162_rn(gain[v].z * xr[v].z * inv, gain[v].w * xr[v].w * inv);
-                uint2 pk;
-                pk.x = *reinterpret_cast<uint32_t*>(&lo);
-                pk.y = *reinterpret_cast<uint32_t*>(&hi);
-                reinterpret_cast<uint2*>(out + (size_t)row * H)[c] = pk;
-            }
+            if (c < H4)
+                store4(out + (size_t)row * H, c, gain[v].x * xr[v].x * inv, gain[v].y * xr[v].y * inv, gain[v].z * xr[v].z * inv,
+                       gain[v].w * xr[v].w * inv);
         }
 #pragma unroll
         for (int v = 0; v < VPT; ++v) {
@@ -261,8 +269,8 @@ VCB_API int vcb_add_rmsnorm(float* resid, const void* delta, int delta_dtype, in
         cudaFuncSetAttribute(add_rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         opted_in = true;
     }
-    const bool vec = H % 4 == 0 && out_dtype == VCB_BF16 && (S == 0 || delta_dtype == VCB_F32) && delta_stride % 4 == 0 &&
-                     ((uintptr_t)resid % 16 == 0) && ((uintptr_t)delta % 16 == 0) && ((uintptr_t)out % 8 == 0) && H <= 16384;
+    const bool vec = H % 4 == 0 && (S == 0 || delta_dtype == VCB_F32) && delta_stride % 4 == 0 && ((uintptr_t)resid % 16 == 0) &&
+                     ((uintptr_t)delta % 16 == 0) && ((uintptr_t)out % (out_dtype == VCB_BF16 ? 8 : 16) == 0) && H <= 16384;
     if (vec) {
         const int H4 = H / 4;
         int threads = H4 >= 1024 ? 1024 : ((H4 + 31) / 32) * 32;
@@ -274,22 +282,26 @@ VCB_API int vcb_add_rmsnorm(float* resid, const void* delta, int delta_dtype, in
         const int vpt = (H4 + threads - 1) / threads;
         const float* d = (const float*)delta;
         __nv_bfloat16* o = (__nv_bfloat16*)out;
-        if (rows == nullptr && S <= 1 && n_out > 4 * 148 && vpt <= 2) {
+        if (out_dtype == VCB_BF16 && rows == nullptr && S <= 1 && n_out > 4 * 148 && vpt <= 2) {
             const int grid = 2 * 148;   // two blocks of 1024 threads fill an SM
             if (vpt == 1) launch_pdl(add_rmsnorm_stream_kernel<1>, dim3(grid), dim3(threads), 0, stream, resid, d, S, w, w_dtype, eps, o, n_out, H);
             else launch_pdl(add_rmsnorm_stream_kernel<2>, dim3(grid), dim3(threads), 0, stream, resid, d, S, w, w_dtype, eps, o, n_out, H);
             VCB_CHECK_LAUNCH("add_rmsnorm");
             return 0;
         }
-        if (vpt == 1) launch_pdl(add_rmsnorm_vec_kernel<1>, dim3(n_out), dim3(threads), 0, stream, resid, d, S, (size_t)delta_stride, w, w_dtype, eps, o, rows, H);
-        else if (vpt == 2) launch_pdl(add_rmsnorm_vec_kernel<2>, dim3(n_out), dim3(threads), 0, stream, resid, d, S, (size_t)delta_stride, w, w_dtype, eps, o, rows, H);
-        else launch_pdl(add_rmsnorm_vec_kernel<4>, dim3(n_out), dim3(threads), 0, stream, resid, d, S, (size_t)delta_stride, w, w_dtype, eps, o, rows, H);
+        auto launch = [&](auto* to) {
+            using T = std::remove_pointer_t<decltype(to)>;
+            auto kern = vpt == 1 ? add_rmsnorm_vec_kernel<1, T> : vpt == 2 ? add_rmsnorm_vec_kernel<2, T> : add_rmsnorm_vec_kernel<4, T>;
+            launch_pdl(kern, dim3(n_out), dim3(threads), 0, stream, resid, d, S, (size_t)delta_stride, w, w_dtype, eps, to, rows, H);
+        };
+        if (out_dtype == VCB_BF16) launch(o);
+        else launch((float*)out);
         VCB_CHECK_LAUNCH("add_rmsnorm");
         return 0;
     }
     const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
-    add_rmsnorm_kernel<<<n_out, threads, smem, stream>>>(resid, delta, delta_dtype, S, (size_t)delta_stride, w, w_dtype,
-                                                         eps, out, out_dtype, rows, H);
+    launch_pdl(add_rmsnorm_kernel, dim3(n_out), dim3(threads), smem, stream, resid, delta, delta_dtype, S, (size_t)delta_stride, w, w_dtype,
+               eps, out, out_dtype, rows, H);
     VCB_CHECK_LAUNCH("add_rmsnorm");
     return 0;
 }
@@ -587,6 +599,17 @@ __global__ __launch_bounds__(256) void qknorm_rope_kvwrite_hd128_kernel(
     constexpr int hd = 128, half = 64;
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int heads_total = nh + (has_kv ? 2 * nkv : 0);
+    pdl_trigger();
+    float gq[4] = {1.f, 1.f, 1.f, 1.f}, gk[4] = {1.f, 1.f, 1.f, 1.f};   // gains of this lane's four elements
+    if (use_norm) {
+        gq[0] = load_as_f32(qw, w_dtype, 2 * lane); gq[1] = load_as_f32(qw, w_dtype, 2 * lane + 1);
+        gq[2] = load_as_f32(qw, w_dtype, half + 2 * lane); gq[3] = load_as_f32(qw, w_dtype, half + 2 * lane + 1);
+        if (has_kv) {
+            gk[0] = load_as_f32(kw, w_dtype, 2 * lane); gk[1] = load_as_f32(kw, w_dtype, 2 * lane + 1);
+            gk[2] = load_as_f32(kw, w_dtype, half + 2 * lane); gk[3] = load_as_f32(kw, w_dtype, half + 2 * lane + 1);
+        }
+    }
+    pdl_wait();
     int pos = positions[t];
     if (pos < 0 || pos >= max_pos) {
         if (threadIdx.x == 0) atomicOr(status, VCB_STATUS_BAD_POSITION);
@@ -598,15 +621,6 @@ __global__ __launch_bounds__(256) void qknorm_rope_kvwrite_hd128_kernel(
     if (slot >= 0 && slot / page_size >= num_pages) {
         if (threadIdx.x == 0) atomicOr(status, VCB_STATUS_BAD_PAGE);
         slot = -1;
-    }
-    float gq[4] = {1.f, 1.f, 1.f, 1.f}, gk[4] = {1.f, 1.f, 1.f, 1.f};   // gains of this lane's four elements
-    if (use_norm) {
-        gq[0] = load_as_f32(qw, w_dtype, 2 * lane); gq[1] = load_as_f32(qw, w_dtype, 2 * lane + 1);
-        gq[2] = load_as_f32(qw, w_dtype, half + 2 * lane); gq[3] = load_as_f32(qw, w_dtype, half + 2 * lane + 1);
-        if (has_kv) {
-            gk[0] = load_as_f32(kw, w_dtype, 2 * lane); gk[1] = load_as_f32(kw, w_dtype, 2 * lane + 1);
-            gk[2] = load_as_f32(kw, w_dtype, half + 2 * lane); gk[3] = load_as_f32(kw, w_dtype, half + 2 * lane + 1);
-        }
     }
     const __nv_bfloat16* row = qkv + (size_t)t * heads_total * hd;
     // six heads a round (the 48 heads of the 8B shape in one round of eight warps): their loads are all issued
@@ -668,7 +682,7 @@ VCB_API int vcb_qknorm_rope_kvwrite(const void* qkv, int in_dtype, int S, long l
                   nh, nkv, page_size, S);
     if (hd == 128 && rot_dim == hd && !interleaved && in_dtype == VCB_BF16 && out_dtype == VCB_BF16 && S == 1 && ((uintptr_t)qkv % 4 == 0) &&
         ((uintptr_t)q_out % 4 == 0) && ((uintptr_t)pages % 4 == 0)) {
-        qknorm_rope_kvwrite_hd128_kernel<<<T, 256, 0, stream>>>(
+        launch_pdl(qknorm_rope_kvwrite_hd128_kernel, dim3(T), dim3(256), 0, stream,
             (const __nv_bfloat16*)qkv, qw, kw, w_dtype, use_norm, eps, cos_sin, max_pos, positions, slot_map,
             (__nv_bfloat16*)q_out, (__nv_bfloat16*)pages, page_stride, page_size, num_pages, nh, nkv, has_kv, status);
         VCB_CHECK_LAUNCH("qknorm_rope_kvwrite");
