@@ -130,3 +130,15 @@ def test_captured_steps_send_crowds_of_single_tokens_to_the_blocks_that_walk_the
     assert A.stream_pays(plan(64, 512), 8) and not A.stream_pays(plan(64, 4096), 8)    # known contexts: as before
     monkeypatch.setattr(A, "STREAM_DECODE", 0)
     assert not A.stream_pays(captured(64), 8)
+
+
+def test_single_tokens_join_long_portions():
+    """Single tokens run as portions of one token where the longest of their key ranges is no longer than what every block of
+    the prompt kernel has to walk anyway; never in steps without portions, or without single tokens."""
+    from vllm_cpp_b200.parts.attention import singles_join_portions
+    assert singles_join_portions([1] * 24 + [2024], [1600] * 24 + [3024], 8, 32)
+    assert not singles_join_portions([1] * 24 + [300], [1600] * 24 + [300], 8, 32)      # little beside the single tokens
+    assert not singles_join_portions([1, 2024], [30000, 2024], 8, 32)                   # one key range longer than the rest
+    assert not singles_join_portions([1] * 24, [1600] * 24, 8, 32)
+    assert not singles_join_portions([2024], [3024], 8, 32)
+    assert not singles_join_portions([0, 0, 2024], [0, 0, 3024], 8, 32)                 # empty slots are nobody's tokens

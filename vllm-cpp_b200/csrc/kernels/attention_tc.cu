@@ -339,10 +339,9 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
 
     tl_mark(VCB_TL_ATTN_TC, 0);
     pdl_trigger();
-    pdl_wait();   // the queries and the newest keys come from the kernel before this one
-    tl_mark(VCB_TL_ATTN_TC, 1);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (base & 1023u) {                  // the layout below needs the alignment asked for above
+        pdl_wait();
         if (tid == 0) atomicOr(a.status, VCB_STATUS_BAD_LAYOUT);
         return;
     }
@@ -397,6 +396,8 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();   // the queries and the newest keys come from the kernel before this one
+    tl_mark(VCB_TL_ATTN_TC, 1);
     const uint32_t tmem_base = *tmem_holder;
     const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 2 * BNK;   // S, S, O
     const uint32_t tmem_q = tmem_base + 256;      // (IN_TMEM)
