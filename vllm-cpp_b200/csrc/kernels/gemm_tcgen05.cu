@@ -184,9 +184,9 @@ __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f 
 // Epilogue of a product whose weight rows alternate gate_i, up_i: lane 2i holds gate_i, lane 2i+1 up_i of the same tokens.
 // v: CHUNK token columns of this lane's row m (M: where the rows end); writes out[token][m / 2].  Of every two tokens the even
 // lane takes the first and the odd lane the second, so one shuffle and one SiLU a lane serve two columns; lanes two apart
-// then swap, so that each holds two neighbouring features of one of four tokens and stores them in one word.  (A SiLU a column
-// in both lanes and a 16-bit store a column in the even ones were slower than the unit's products: 19,456 rows of 2,560, 911
-// tokens 106.2 us then, 79.5 now; 24,576 of 4,096, 256 tokens 74.3 and 55.5, 2,048 tokens 280.8 and 265.9.)
+// then swap, so that each holds two neighbouring features of one of four tokens and stores them in one word.  (With a SiLU a column
+// in both lanes and a 16-bit store a column in the even ones, and the unit shapes that paid then: 19,456 rows of 2,560, 911 tokens 88.7
+// us, 74.5 now; 24,576 of 4,096, 256 tokens 62.9 and 56.6, 2,048 tokens 282 and 266.)
 // Every lane of the warp must call it.
 template <int CHUNK>
 __device__ __forceinline__ void swiglu_store(uint32_t (*v)[16], __nv_bfloat16* out, long long ldc, int m, int M, int n_first,
@@ -272,7 +272,8 @@ __device__ __forceinline__ void xielu_store(const uint32_t (&v)[CHUNK / 16][16],
 }
 
 // A chunk's sums after an activation (gemm_act), 32-bit or bfloat16.  A last chunk that is not whole stores under a predicate a
-// column, nothing else: with the activation behind each column's branch it took a product 6 to 13 us longer than a whole one.
+// column, nothing else.  (Against the activation behind each column's branch and 16 bits a lane, with the unit shapes chosen anew: 6,144
+// features of 2,560 lanes, 911 tokens, bfloat16 26.8 -> 24.0 us; 2,560 of 9,728 in three k-slices 41.5 -> 40.0.)
 template <int CHUNK>
 __device__ __forceinline__ void plain_store(const uint32_t (&v)[CHUNK / 16][16], void* out, int out_dtype, size_t at, long long ldc, int m, int M,
                                             int t0, int N, int lane, int act) {
@@ -1176,32 +1177,32 @@ int launch_shape(int shape, const void* W, const void* X, GemmArgs g, long long 
 // from L2); drain is a unit's epilogue, hidden behind the next unit's products only where there is a second accumulator, and
 // then only if those take longer (short K); ragged is what a last chunk of tokens that is not whole adds.  The epilogues differ
 // so much that each kind has numbers of its own.
-// Fitted to every shape, launches one behind the other with weights from HBM: plain and SiLU-gate at 627 and 1,330 sizes (1,024 to
-// 34,816 features, 130 to 4,096 tokens, K of 256 to 9,728), the others at 3,686 (heads 1,440).  Taken by the estimate the products
-// are on average 0.5 % (plain), 0.3 (SiLU-gate), 1.3 (k-slices), 0.3 (xIELU) and 1.0 (heads) from the best shape; by the numbers
-// that fitted the first two epilogues before they shared columns between lanes, 3.9 and 1.3 %, and up to 48 (1,024 features of 256
-// lanes, 911 tokens).  By whole rounds of token columns, the rule before the estimate: 6.8, 5.1, 11.8, 2.1 and 4.1 %.
+// Fitted to every shape, launches one behind the other with weights from HBM: plain, SiLU-gate and k-slices at 1,330, 627 and 936
+// sizes (1,024 to 34,816 features, 130 to 4,096 tokens, K of 256 to 9,728), the others at 3,686 (heads 1,440).  Taken by the
+// estimate the products are on average 0.5 % (plain), 0.3 (SiLU-gate), 0.4 (k-slices), 0.3 (xIELU) and 1.0 (heads) from the best
+// shape; by numbers fitted to single launches and to the epilogues before they shared columns between lanes, 3.9 %, 1.3 and 4.0, and up
+// to 48 (1,024 features of 256 lanes, 911 tokens).
 enum Epilogue { EPI_PLAIN = 0, EPI_PARTIAL, EPI_GATE, EPI_XIELU, EPI_HEADS, EPI_COUNT };
 struct UnitTime { float k_block, busy, start, drain, once, ragged; };      // k_block 0: not taken
 struct UnitShape { int shape, tiles, tokens, blocks, chunk; UnitTime time[EPI_COUNT]; };
 const UnitShape UNIT_SHAPES[] = {
     {SHAPE_PAIR, 2, 256, 2, 64,
-     {{0.264f, 0.28f, 1.5f, 0.4f, 4.6f, 0.2f}, {0.286f, 0.35f, 2.0f, 0.0f, 10.4f, 6.2f}, {0.276f, 0.28f, 0.9f, 3.3f, 1.6f, 0.1f},
+     {{0.264f, 0.28f, 1.5f, 0.4f, 4.6f, 0.2f}, {0.255f, 0.38f, 1.3f, 3.0f, 2.5f, 0.1f}, {0.276f, 0.28f, 0.9f, 3.3f, 1.6f, 0.1f},
       {0.280f, 0.24f, 2.3f, 4.0f, 7.8f, 0.0f}, {0.254f, 0.16f, 8.6f, 8.6f, 11.4f, 0.0f}}},
     {SHAPE_PAIR_TOKENS + 224, 2, 224, 2, 32,
-     {{0.268f, 0.21f, 1.3f, 3.0f, 1.7f, 0.0f}, {0.281f, 0.29f, 1.4f, 2.3f, 8.7f, 1.0f}, {0.274f, 0.22f, 0.9f, 3.5f, 1.4f, 0.1f},
+     {{0.268f, 0.21f, 1.3f, 3.0f, 1.7f, 0.0f}, {0.248f, 0.33f, 1.3f, 0.0f, 5.0f, 0.3f}, {0.274f, 0.22f, 0.9f, 3.5f, 1.4f, 0.1f},
       {0.277f, 0.20f, 2.5f, 4.2f, 6.8f, 0.0f}, {0.258f, 0.07f, 8.5f, 4.5f, 13.2f, 0.0f}}},
     {SHAPE_PAIR_TOKENS + 192, 2, 192, 2, 64,
-     {{0.268f, 0.16f, 1.0f, 1.9f, 2.9f, 0.4f}, {0.292f, 0.12f, 1.4f, 0.0f, 10.4f, 6.1f}, {0.278f, 0.16f, 0.7f, 2.6f, 2.1f, 0.3f},
+     {{0.268f, 0.16f, 1.0f, 1.9f, 2.9f, 0.4f}, {0.264f, 0.19f, 0.8f, 2.4f, 3.1f, 0.4f}, {0.278f, 0.16f, 0.7f, 2.6f, 2.1f, 0.3f},
       {0.284f, 0.14f, 1.8f, 3.0f, 8.5f, 0.4f}, {0.283f, 0.00f, 6.2f, 9.2f, 8.5f, 0.0f}}},
     {SHAPE_PAIR_TOKENS + 160, 2, 160, 2, 32,
-     {{0.280f, 0.11f, 0.8f, 2.3f, 2.4f, 0.1f}, {0.287f, 0.14f, 0.9f, 1.8f, 9.1f, 1.5f}, {0.282f, 0.11f, 0.6f, 2.7f, 2.0f, 0.2f},
+     {{0.280f, 0.11f, 0.8f, 2.3f, 2.4f, 0.1f}, {0.264f, 0.18f, 0.6f, 2.2f, 3.0f, 0.2f}, {0.282f, 0.11f, 0.6f, 2.7f, 2.0f, 0.2f},
       {0.284f, 0.14f, 1.5f, 3.2f, 7.7f, 0.0f}, {0.274f, 0.00f, 5.5f, 3.1f, 13.7f, 0.0f}}},
     {SHAPE_N256, 1, 256, 1, 64,
-     {{0.309f, 0.26f, 0.9f, 3.0f, 0.8f, 0.1f}, {0.348f, 0.30f, 2.2f, 0.0f, 8.8f, 4.4f}, {0.315f, 0.26f, 0.5f, 3.4f, 0.4f, 0.2f},
+     {{0.309f, 0.26f, 0.9f, 3.0f, 0.8f, 0.1f}, {0.296f, 0.37f, 1.7f, 3.0f, 0.6f, 0.0f}, {0.315f, 0.26f, 0.5f, 3.4f, 0.4f, 0.2f},
       {0.349f, 0.14f, 2.3f, 4.3f, 5.8f, 0.0f}, {0.322f, 0.05f, 8.0f, 7.7f, 10.7f, 0.0f}}},
     {SHAPE_N128, 1, 128, 1, 64,
-     {{0.240f, 0.14f, 0.7f, 1.5f, 2.5f, 0.2f}, {}, {0.247f, 0.13f, 0.4f, 2.0f, 1.6f, 0.2f},
+     {{0.240f, 0.14f, 0.7f, 1.5f, 2.5f, 0.2f}, {0.237f, 0.18f, 0.7f, 2.0f, 2.2f, 0.2f}, {0.247f, 0.13f, 0.4f, 2.0f, 1.6f, 0.2f},
       {0.254f, 0.16f, 1.1f, 2.6f, 7.1f, 0.0f}, {0.261f, 0.00f, 3.5f, 6.7f, 7.4f, 0.0f}}},
     {SHAPE_M256_N256, 2, 256, 1, 64,
      {{0.543f, 0.26f, 0.0f, 4.5f, 2.8f, 0.3f}, {}, {0.537f, 0.30f, 0.0f, 5.6f, 2.7f, 0.2f},
