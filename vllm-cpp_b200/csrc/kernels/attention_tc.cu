@@ -396,6 +396,16 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // What no kernel of the step writes -- the work items, the entries' lengths, the block tables -- is read before the wait:
+    // the block's first unit, and the first page of its keys (each a round trip to memory behind another).
+    Unit u;
+    bool has = read_unit<OPT>(a, (int)blockIdx.x, u);
+    const int pages_per_tile = BNK / ps;
+    auto first_page = [&](const Unit& w) {      // a loading lane's page id for the first tile of a unit (see page_of below)
+        const int pl = lane & 7, pb = tile_pb0(w, 0, pages_per_tile) + pl;
+        return (lane < 16 && pl < pages_per_tile && pb < tile_pb_hi(w, 0, ps)) ? a.block_table[(size_t)w.bt_row * a.max_blocks + pb] : -1;
+    };
+    int next_page = warp == 0 && has ? first_page(u) : -1;
     pdl_wait();   // the queries and the newest keys come from the kernel before this one
     tl_mark(VCB_TL_ATTN_TC, 1);
     const uint32_t tmem_base = *tmem_holder;
@@ -407,7 +417,6 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
         // one go: the K tile two ahead of the V tile, so that one wait, one round of byte counts and one divergent
         // copy instruction serve both (a call of its own per tile cost this warp 1,000 clocks, of which the copies
         // themselves were a third, and made it the slowest role of the block). ----
-        const int pages_per_tile = BNK / ps;
         const int groups_page = ps / 8;
         const int parts = a.one_row ? 1 : 2;
         const int groups_kv = a.one_row ? 0 : a.nkv * groups_page;   // groups of 8 rows from a page's K to its V
@@ -418,15 +427,7 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
         int t0 = 0;
         TlRole tl;
         tl.begin(VCB_TL_ATTN_TC, 0, lane == 0);
-        Unit u;
         int unit = (int)blockIdx.x;
-        bool has = read_unit<OPT>(a, unit, u);
-        // this lane's page id for the first tile of the unit (see page_of below)
-        auto first_page = [&](const Unit& w) {
-            const int pb = tile_pb0(w, 0, pages_per_tile) + pl;
-            return (lane < 16 && pl < pages_per_tile && pb < tile_pb_hi(w, 0, ps)) ? a.block_table[(size_t)w.bt_row * a.max_blocks + pb] : -1;
-        };
-        int next_page = has ? first_page(u) : -1;
         for (int seq = 0; unit >= 0 && ok; ++seq) {
             // The unit after this one.  Its number is asked for when this one has four tiles to go -- not earlier, or
             // the blocks that start first would take the whole queue while they still have their long first units
@@ -556,9 +557,7 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
             int t0 = 0, done = 0;
             TlRole tl;
             tl.begin(VCB_TL_ATTN_TC, 1, true);
-            Unit u;
             int unit = (int)blockIdx.x;
-            bool has = read_unit<OPT>(a, unit, u);
             for (int seq = 0; unit >= 0 && ok; unit = next_unit(seq, u), has = unit >= 0, ++seq) {
                 if (!has) continue;
                 // The rows have read the output of the unit before and written this unit's queries.
@@ -620,12 +619,10 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
     } else if (WIDE && warp >= NTHREADS / 32) {
         // ---- wide rows: the keys, a stage (a tile's keys of one KV head) in turn for each of these warps, a lane a page ----
         const int me = warp - NTHREADS / 32;
-        const int pages_per_tile = BNK / ps, groups_page = ps / 8;
+        const int groups_page = ps / 8;
         bool ok = true;
         int g0 = 0, armed = -1;     // stages of the units before; the last stage this warp has asked for
-        Unit u;
         int unit = (int)blockIdx.x;
-        bool has = read_unit<OPT>(a, unit, u);
         for (int seq = 0; unit >= 0 && ok; unit = next_unit(seq, u), has = unit >= 0, ++seq) {
             if (!has) continue;
             const int* bt = a.block_table + (size_t)u.bt_row * a.max_blocks;
@@ -721,9 +718,7 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
 #pragma unroll
             for (int c = 0; c < (WIDE ? 1 : CH); ++c) qv[c] = mine ? *reinterpret_cast<const uint4*>(src + c * 8) : make_uint4(0, 0, 0, 0);
         };
-        Unit u;
         int unit = (int)blockIdx.x, seq = 0;
-        bool has = read_unit<OPT>(a, unit, u);
         ask_query(u, has);
         while (unit >= 0 && ok) {
             if (!has) {
