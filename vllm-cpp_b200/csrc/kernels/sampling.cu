@@ -30,14 +30,29 @@ __device__ __forceinline__ float uniform01(unsigned long long key, unsigned int 
     return ((float)(bits >> 41) + 0.5f) * (1.0f / 8388608.0f);
 }
 
-// uniform01 lies in [2^-24, 1 - 2^-24], so -log(-log(u)) lies between these: a score that cannot reach the best draw so
-// far even with the largest of them needs no logarithms (rounding keeps the order, so the token is the same)
-constexpr float GUMBEL_MAX = 16.75f, GUMBEL_MIN = -2.85f;
+// uniform01 lies in [2^-24, 1 - 2^-24], so -log(-log(u)) is no more than this: a score that cannot reach the best draw so
+// far even with it needs no logarithms (rounding keeps the order, so the token is the same)
+constexpr float GUMBEL_MAX = 16.75f;
+
+// Whether score s with uniform u may draw as much as `best`, which takes a hash and an exponential where the draw itself takes two
+// logarithms more: -log(u) >= 1 - u, so the draw is at most s - log(1 - u).  What is let through in vain costs time only; the
+// margins (a hundredth of the exponential, 1e-3 and five units of 2^-23 of `best`) are far above what rounding adds to either side.
+// Infinities and NaN are let through.
+__device__ __forceinline__ bool may_draw(float s, float u, float best) {
+    const float d = best - s - fmaf(fabsf(best), 6e-7f, 1e-3f);
+    return !(1.f - u > 1.01f * __expf(-d));
+}
 
 // order-preserving map float -> uint32
 __device__ __forceinline__ unsigned int ordered_key(float f) {
     const unsigned int u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// the score of a key; no score is less than minus infinity (keys of NaN below it)
+__device__ __forceinline__ float score_of(unsigned int key) {
+    const float f = __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+    return f == f ? f : -CUDART_INF_F;
 }
 
 __device__ __forceinline__ double block_sum_f64(double v, double* scratch /* 33 */) {
@@ -153,12 +168,13 @@ __global__ __launch_bounds__(1024) void sample_kernel(const float* __restrict__ 
     }
 
     const unsigned long long key = mix64(((unsigned long long)p.seed_lo << 32) | (unsigned long long)p.step);
-    float zbest = -CUDART_INF_F;
-    int zi = 0x7fffffff;
+    float zbest = m - logf(-logf(uniform01(key, (unsigned int)best_i)));       // the largest score's draw, which all others have to reach
+    int zi = best_i;
     for (int i = threadIdx.x; i < V; i += blockDim.x) {
         const float s = score_at(lg, counts, p.repeat_penalty, inv_t, i);
-        if (ordered_key(s) < cut) continue;
+        if (ordered_key(s) < cut || s + GUMBEL_MAX < zbest) continue;
         const float u = uniform01(key, (unsigned int)i);
+        if (!may_draw(s, u, zbest)) continue;
         const float zv = s - logf(-logf(u));
         if (zv > zbest || (zv == zbest && i < zi)) { zbest = zv; zi = i; }
     }
@@ -175,8 +191,11 @@ __global__ __launch_bounds__(1024) void sample_kernel(const float* __restrict__ 
 // on by NT thresholds a pass: the first pass puts them at distances below the maximum, where the mass of a softmax lies,
 // later ones spread them evenly over the remaining range of ordered keys.  Once the range holds at most CAND scores, every
 // block takes the cluster's list of them, ranks it, and reads the cut off the running sum -- in a model's logits after the
-// first pass.  All sums are taken in a fixed order, so equal logits give equal tokens.  64 rows of 151,936 with penalty, temperature and nucleus: 1,620 us with a block a row, 71 here; one row
-// 27 us from a cold L2.
+// first pass.  All sums are taken in a fixed order, so equal logits give equal tokens.
+// The passes over a block's scores are bound by instructions (128 a score before, of which every score's ordered key, eight
+// predicated sums and a comparison of places were most), so a score that reaches no threshold is left at one comparison of floats.
+// 64 rows of 151,936 with penalty, temperature and nucleus: 1,620 us with a block a row, 56 here (71 with keys and sums for every
+// score); with a temperature alone 41 (56 with two logarithms for every score near the maximum).
 namespace cg = cooperative_groups;
 constexpr size_t CLUSTER_MAX_SMEM = 192 * 1024;      // beside ClusterShared (18 KB)
 constexpr int CL_THREADS = 512, CL_WARPS = CL_THREADS / 32, CL_BLOCKS = 8, NT = 7, CAND = 1024;
@@ -262,11 +281,13 @@ __device__ bool cut_from_list(cg::cluster_group& cluster, ClusterShared& sh, con
     if (tid == 0) sh.n_cand = 0;
     __syncthreads();
     const float4* scores4 = reinterpret_cast<const float4*>(scores);
+    const float least = score_of(lo);
     for (int q = tid; q < (n + 3) / 4; q += CL_THREADS) {
         const float4 f = scores4[q];       // (lanes beyond n: the buffer holds a multiple of 4)
         const float e[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
+            if (e[j] < least) continue;
             const unsigned int k = ordered_key(e[j]);
             if (k >= lo && k < hi && 4 * q + j < n) {
                 const int at = atomicAdd(&sh.n_cand, 1);
@@ -387,12 +408,14 @@ __global__ __launch_bounds__(CL_THREADS, 2) void sample_cluster_kernel(const flo
                     f[3] = penalised(f[3], c[u].w, p.repeat_penalty);
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    f[j] *= inv_t;
-                    const int i = i0 + 4 * q + j;
-                    if (f[j] > best || (f[j] == best && i < best_i)) { best = f[j]; best_i = i; }
-                }
+                for (int j = 0; j < 4; ++j) f[j] *= inv_t;
                 scores4[q] = make_float4(f[0], f[1], f[2], f[3]);
+                // (a thread's places ascend: only more than its best so far, or its first score, takes the lead)
+                const float most = fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3]));
+                if (most > best || (most == best && best_i == 0x7fffffff)) {
+                    best = most;
+                    best_i = i0 + 4 * q + (f[0] == most ? 0 : f[1] == most ? 1 : f[2] == most ? 2 : 3);
+                }
             }
         }
     } else {
@@ -401,6 +424,7 @@ __global__ __launch_bounds__(CL_THREADS, 2) void sample_cluster_kernel(const flo
             if (s > best || (s == best && i0 + i < best_i)) { best = s; best_i = i0 + i; }
             scores[i] = s;
         }
+        if (tid < 4 && n + tid < (n + 3) / 4 * 4) scores[n + tid] = -CUDART_INF_F;      // no mass where there is no score
     }
     cluster_argmax(cluster, sh, 0, best, best_i);      // (its barriers order the scores too)
     const float m = best;
@@ -426,20 +450,33 @@ __global__ __launch_bounds__(CL_THREADS, 2) void sample_cluster_kernel(const flo
                 double v[NT + 1];
 #pragma unroll
                 for (int j = 0; j <= NT; ++j) v[j] = 0.0;
+                // Bound by instructions: a score below all thresholds costs its exponential and one sum (the first pass) or a
+                // comparison (later ones), and a branch each for the thresholds it reaches, most often none.
+                const float least = score_of(t[0]);
+                auto above = [&](float x, double e) {
+                    const unsigned int k = ordered_key(x);
+                    if (k >= t[0] && k < hi) {
+                        if (pass > 0) v[NT] += e;
+                        v[0] += e;
+                        if (k >= t[1]) { v[1] += e;
+                        if (k >= t[2]) { v[2] += e;
+                        if (k >= t[3]) { v[3] += e;
+                        if (k >= t[4]) { v[4] += e;
+                        if (k >= t[5]) { v[5] += e;
+                        if (k >= t[6]) v[6] += e; } } } } }
+                    }
+                };
                 for (int q = tid; q < (n + 3) / 4; q += CL_THREADS) {
                     const float4 f = scores4[q];
                     const float s[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        const unsigned int k = ordered_key(s[c]);
-                        if ((pass == 0 || (k >= t[0] && k < hi)) && 4 * q + c < n) {
+                        if (pass == 0) {
                             const double e = (double)expf(s[c] - m);
                             v[NT] += e;
-                            if (k >= t[0]) {
-#pragma unroll
-                                for (int j = 0; j < NT; ++j)
-                                    if (k >= t[j]) v[j] += e;
-                            }
+                            if (!(s[c] < least)) above(s[c], e);
+                        } else if (!(s[c] < least) && 4 * q + c < n) {
+                            above(s[c], (double)expf(s[c] - m));
                         }
                     }
                 }
@@ -461,17 +498,18 @@ __global__ __launch_bounds__(CL_THREADS, 2) void sample_cluster_kernel(const flo
             }
         }
         const unsigned long long key = mix64(((unsigned long long)p.seed_lo << 32) | (unsigned long long)p.step);
-        const float floor_z = m + GUMBEL_MIN;      // the row's largest score draws at least this
-        best = -CUDART_INF_F;
-        best_i = 0x7fffffff;
+        best = m - logf(-logf(uniform01(key, (unsigned int)best_i)));      // the largest score's draw, which all others have to reach
+        const float least = score_of(cut);
         for (int q = tid; q < (n + 3) / 4; q += CL_THREADS) {
             const float4 f = scores4[q];
             const float s[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int i = i0 + 4 * q + j;
-                if (4 * q + j >= n || ordered_key(s[j]) < cut || s[j] + GUMBEL_MAX < fmaxf(floor_z, best)) continue;
-                const float zv = s[j] - logf(-logf(uniform01(key, (unsigned int)i)));
+                if (s[j] < least || s[j] + GUMBEL_MAX < best || 4 * q + j >= n || ordered_key(s[j]) < cut) continue;
+                const float u = uniform01(key, (unsigned int)i);
+                if (!may_draw(s[j], u, best)) continue;
+                const float zv = s[j] - logf(-logf(u));
                 if (zv > best || (zv == best && i < best_i)) { best = zv; best_i = i; }
             }
         }
@@ -507,7 +545,9 @@ __global__ __launch_bounds__(512) void sample_part_kernel(const float* __restric
         float s = score_at(lg, counts, p.repeat_penalty, inv_t, i);
         if (!greedy) {
             if (s + GUMBEL_MAX < best) continue;
-            s -= logf(-logf(uniform01(key, (unsigned int)i)));
+            const float u = uniform01(key, (unsigned int)i);
+            if (!may_draw(s, u, best)) continue;
+            s -= logf(-logf(u));
         }
         if (s > best || (s == best && i < best_i)) { best = s; best_i = i; }
     }
