@@ -66,3 +66,26 @@ def test_rows_of_logits_a_step_computes():
     assert r.rows_capacity([entry(60)]) == 1
     assert r.rows_capacity([entry(600), entry(700, slot=1, want="none")]) == 1
     assert fake_runner(graphs=False).rows_capacity(singles) == 5
+
+
+def test_portions_pad_to_half_way_steps_from_64_on():
+    r = fake_runner()
+    assert [r.portion_size([entry(n)]) for n in (64, 65, 96, 97, 129, 193, 257, 385)] == [64, 96, 96, 128, 192, 256, 384, 512]
+
+
+def test_portions_whose_launches_hide_run_kernel_by_kernel():
+    """A 32-bit engine's portions beyond its limit are not padded: neither alone nor beside single tokens."""
+    r = fake_runner()
+    r.capture_limit = 44
+    assert r.portion_size([entry(44)]) == 64 and r.portion_size([entry(45)]) is None
+    singles = [entry(1, slot=i) for i in range(5)]
+    assert r.mixed_size(singles + [entry(39, slot=9)]) == (8, 64) and r.mixed_size(singles + [entry(40, slot=9)]) is None
+    assert r.capture_size(singles) == 8                     # single tokens stay captured
+    from vllm_cpp_b200.engine.step import _launches_hide_from
+    spec = lambda *shape, role="matrix": types.SimpleNamespace(shape=shape, role=role)
+    part = lambda *specs, **kw: types.SimpleNamespace(tensor_specs=lambda: list(specs), **kw)
+    layer = types.SimpleNamespace(parts=dict(a=part(spec(6144, 2560), spec(2560, role="vector")), b=part(spec(9728 * 3, 2560), spec(4096, 2560)),
+                                             c=part(spec(100, 1000, 1000), spec(1 << 20, 1 << 10), top=2)))
+    model = types.SimpleNamespace(layers=[layer], order=[types.SimpleNamespace(layer=0)] * 36)
+    assert 30 < _launches_hide_from(model) < 60
+    assert _launches_hide_from(types.SimpleNamespace()) is None

@@ -1143,6 +1143,7 @@ VCB_API int vcb_gemm_effective_splits(int K, int splits) {
 // The unit shapes that are built: tokens per tile (BN), stages of the ring, 128-feature tiles per unit, accumulators.
 enum GemmShape { SHAPE_N16 = 0, SHAPE_N32, SHAPE_N64, SHAPE_N128, SHAPE_N256, SHAPE_M256_N192, SHAPE_M256_N256, SHAPE_PAIR, SHAPE_M256_N160,
                  SHAPE_COUNT,
+                 SHAPE_N96 = 96,               // units of up to 96 tokens
                  SHAPE_PAIR_TOKENS = 1000,     // + 160, 192 or 224: pairs with that many tokens a unit
                  SHAPE_ROWS = 2000 };          // + 8 to 128 in steps of 8: units of that many features and up to 128 tokens
 
@@ -1151,12 +1152,13 @@ int launch_shape(int shape, const void* W, const void* X, GemmArgs g, long long 
                  cudaStream_t stream) {
     if (shape > SHAPE_ROWS && shape <= SHAPE_ROWS + BM && shape % 8 == 0) {
         g.unit_rows = shape - SHAPE_ROWS;
-        shape = g.N <= 16 ? SHAPE_N16 : g.N <= 32 ? SHAPE_N32 : g.N <= 64 ? SHAPE_N64 : SHAPE_N128;
+        shape = g.N <= 16 ? SHAPE_N16 : g.N <= 32 ? SHAPE_N32 : g.N <= 64 ? SHAPE_N64 : g.N <= 96 ? SHAPE_N96 : SHAPE_N128;
     }
     switch (shape) {
         case SHAPE_N16: return launch<16, 8, 1, 2>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_N32: return launch<32, 8, 1, 2>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_N64: return launch<64, 8, 1, 2>(W, X, g, ldw, ldx, splits, stream);
+        case SHAPE_N96: return launch<96, 7, 1, 2>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_N128: return launch<128, 6, 1, 2>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_N256: return launch<256, 4, 1, 2>(W, X, g, ldw, ldx, splits, stream);
         case SHAPE_M256_N192: return launch<192, 3, 2, 1>(W, X, g, ldw, ldx, splits, stream);
@@ -1220,6 +1222,7 @@ int choose_shape(int M, int N, int K, int splits, Epilogue epilogue) {
     if (N <= 16) return SHAPE_N16;
     if (N <= 32) return SHAPE_N32;
     if (N <= 64) return SHAPE_N64;
+    if (N <= 96) return SHAPE_N96;
     if (N <= 128) return SHAPE_N128;
     const bool pairs = pairs_mode() != 0 && M >= 2 * BM;
     if (pairs && pairs_mode() == 2) return SHAPE_PAIR;

@@ -179,13 +179,26 @@ class StepContext:
         return self._plans[key]
 
 
+def _launches_hide_from(model) -> int | None:
+    """Tokens beyond which the 32-bit products of a portion take the GPU half as long again as the host needs to launch a layer:
+    some 150 us a run of the execution order, against 40 TFLOP/s.  Experts, of which a token meets a few, do not count."""
+    weights = 0
+    for run in getattr(model, "order", ()):
+        for part in model.layers[run.layer].parts.values():
+            if not hasattr(part, "top"):
+                weights += sum(s.shape[0] * s.shape[1] for s in part.tensor_specs() if s.role == "matrix" and len(s.shape) == 2 and min(s.shape) > 0)
+    return max(1, int(1.5 * 150e-6 * 40e12 * len(model.order) / (2 * weights))) if weights else None
+
+
 class ModelRunner:
     """Owns the model, its device cache, the device-resident block tables and the status word; runs steps."""
 
     GRAPH_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256)
     GRAPH_CONTEXT_BOUNDS = (8192,)      # captured steps are kept per context class: up to 8192 tokens, and beyond
     MAX_GRAPHS = 48                     # captured steps kept; the least recently used one goes when another is captured
-    PORTION_BUCKETS = (16, 32, 64, 128, 256, 512)   # token counts of captured steps that run one prompt portion
+    # token counts of captured steps that run one prompt portion; half-way steps from 64 on, where the rows that are padding
+    # begin to cost what the weights do (8B sizes, 77 tokens padded to 128: 4.31 ms, to 96: 4.07)
+    PORTION_BUCKETS = (16, 32, 64, 96, 128, 192, 256, 384, 512)
     # captured steps of single tokens beside prompt portions: slots for single-token entries, which come first, then
     # MIXED_PORTIONS slots for portions; MIXED_TOKENS are the token rows of the whole step (the products work in
     # token tiles of up to 256: a step padded to 264 rows would cost two tiles)
@@ -228,6 +241,10 @@ class ModelRunner:
         # (a model with a part that reads host-side facts of a step cannot run over padding: its scratch grows on demand)
         if max_step_tokens and self.device.type == "cuda" and getattr(model, "capturable", True):
             self.size_workspace(max_step_tokens)
+        # A captured step pads a portion to its bucket, which hides the host's launches.  32-bit products are bound by
+        # multiply-adds: there a portion that takes the GPU longer than its launches take the host runs kernel by kernel over
+        # its own tokens (201 tokens of the 4B sizes: 51.7 ms padded to 256 and replayed, 48.8 so).
+        self.capture_limit = _launches_hide_from(model) if dtype == torch.float32 and self.cuda_graphs else None
         self.graph_replays = 0
         self.launches_per_graph: dict[tuple, int] = {}
 
@@ -350,6 +367,8 @@ class ModelRunner:
         n = len(e.tokens)
         if n < 2 or n > self.PORTION_BUCKETS[-1] or e.want not in ([], [n - 1]):
             return None
+        if n > (getattr(self, "capture_limit", None) or n):
+            return None
         return next(b for b in self.PORTION_BUCKETS if b >= n)
 
     def mixed_size(self, entries) -> tuple[int, int] | None:
@@ -371,6 +390,8 @@ class ModelRunner:
             if n < 2 or e.want not in ([], [n - 1]):
                 return None
             tokens += n
+        if n_single + tokens > (getattr(self, "capture_limit", None) or n_single + tokens):
+            return None
         singles = next(b for b in self.MIXED_SINGLES if b >= n_single)
         rows = next((b for b in self.MIXED_TOKENS if b >= singles + tokens), None)
         return None if rows is None else (singles, rows)
