@@ -1017,10 +1017,11 @@ int num_sms() {
 // features: an SM's bytes in flight bound it.  Gate and up of 4,096 inner lanes, 24,576 features: 128 tokens 45.6 us with units of
 // 128, 41.8 of 88 (280 units on 148 SMs) and 55.0 of 80 (a third round), 64 tokens 43.6, 38.5 and 52.3; 19,456 of 2,560, 64
 // tokens 27.3, 24.2 of 88, 25.0 of 72; the head, 151,936 of 2,560, 127.7 and 123.7 of 120.  One round gains nothing by it
-// (4,096 features in four k-slices: 9.2 us with 128 units of 128, 9.4 with 148 of 112).
-int choose_unit_rows(int M, int n_tiles, int splits) {
+// (4,096 features in four k-slices: 9.2 us with 128 units of 128, 9.4 with 148 of 112), and units of a few k-blocks lose in a step
+// (the 4B sizes' gate and up in slices of 10, 12 to 16 tokens: 3,149 us with 128 features, 3,217 with 112).
+int choose_unit_rows(int M, int n_tiles, int splits, int kb_per_split) {
     const long long sms = num_sms(), rounds = ((long long)((M + BM - 1) / BM) * splits + sms - 1) / sms;
-    if (n_tiles > 1 || rounds == 1) return BM;
+    if (n_tiles > 1 || rounds == 1 || kb_per_split < 16) return BM;
     for (int rows = 88; rows < BM; rows += 8)
         if ((long long)((M + rows - 1) / rows) * splits <= rounds * sms) return rows;
     return BM;
@@ -1035,7 +1036,7 @@ int launch_maps(const void* W, long long w_rows, const void* X, GemmArgs g, long
     } else {
         // (a tile of a grouped product and a head of the q, k, v epilogue are 128 features)
         if (g.tile_group != nullptr || g.qe.q_out != nullptr) g.unit_rows = BM;
-        else if (g.unit_rows == 0) g.unit_rows = choose_unit_rows(g.M, (g.N + BN - 1) / BN, splits);
+        else if (g.unit_rows == 0) g.unit_rows = choose_unit_rows(g.M, (g.N + BN - 1) / BN, splits, g.kb_per_split);
         g.stages = L::stages(g.unit_rows);
     }
     CUtensorMap mw, mx;

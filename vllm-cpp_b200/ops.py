@@ -883,11 +883,12 @@ def sample_in_clusters(R: int, V: int, no_nucleus: bool) -> bool:
       rows 68 -> 32, 16,384 x 128 111 -> 59, 32,000 x 256 399 -> 131, 151,936 x 64 1,396 -> 111).  Scores like noise, whose cut
       lies among thousands, take several passes: 8,192 x 128 83 -> 184, which is where the line for small vocabularies comes
       from; above it the most that they lose is 16,384 x 296 242 -> 360, for 197 -> 129 with scores as a model's;
-    * without a cut: greedy 151,936 x 64 48 -> 23, 128,256 x 147 77 -> 43; with a temperature 67 -> 66 and 105 -> 110.  Smaller
-      vocabularies lose (100,000 x 72, with a temperature, 46 -> 55; 8,192 x 512, greedy, 18 -> 76), and larger ones, whose
-      clusters no longer fit an SM twice (196,608 x 64, with a temperature, 83 -> 111)."""
+    * without a cut, against dealt blocks, with a temperature and greedy: 151,936 x 32 32 -> 20 and 12 -> 8, x 64 63 -> 39 and 23 -> 14,
+      x 256 188 -> 141 and 76 -> 57; 128,256 x 32 28 -> 18 and 11 -> 7; 100,000 x 32 24 -> 16 and 9.5 -> 6.9, x 128 78 -> 56 and 29 -> 24.
+      Fewer rows (128,256 x 16 14.8 -> 16.6), smaller vocabularies (65,536 x 256 63 -> 84, 100,000 x 256 102 -> 113) and larger ones, whose
+      clusters no longer fit an SM twice (196,608 x 256 242 -> 261), lose."""
     if no_nucleus:
-        return 64 <= R <= 65535 and 120000 <= V <= 192000
+        return (32 <= R <= 65535 and 120000 <= V <= 192000) or (32 <= R <= 128 and 96000 <= V < 120000)
     return V <= 393216 and R <= 65535 and (V >= 16384 or (V >= 8192 and R <= 64))
 
 
