@@ -615,8 +615,7 @@ class ModelRunner:
         dev = torch.zeros(lay.size, dtype=torch.int32, device=self.device)
         staging = StagingRing(lay.size)
         ctx = StepContext(self, lay, dev, static=True)
-        # no context is longer than the positions there are: an engine for short requests has its key ranges in fewer slices
-        ctx.static_max_ctx = min(ctx_bound or self.max_positions, self.max_positions)
+        ctx.static_max_ctx, ctx.static_positions = ctx_bound, self.max_positions
         host = np.zeros(lay.size, dtype=np.int32)
         o = lay.offsets
         for g in range(len(self.tables)):
