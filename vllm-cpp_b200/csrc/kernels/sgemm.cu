@@ -288,13 +288,19 @@ __global__ __launch_bounds__(32 * SEGMENTS, 2) void sgemm_rows_kernel(const floa
 // items (201 rows against 2,560 features of 9,728 lanes: 1,280 blocks) that fill the SMs evenly.  A thread keeps TMR x 4
 // pairs of sums; per four lanes of K it reads TMR + 4 16-byte words for 8 TMR packed multiply-adds.  Tiles lie as in global
 // memory, rows padded by 16 bytes (eight features: eight different groups of four banks), two stages of 32 lanes of K.
+// Four blocks an SM, or three (BLOCKS), whose threads then have 168 registers instead of 128.  What bounds it is the multiply-add
+// pipe, kept waiting by operands in the same register banks.  Over many rounds of blocks four an SM are the better ones, but in 128
+// registers tiles of 56 and 64 rows spill, and where all blocks are resident at once that is not hidden: three an SM with single
+// multiply-adds take 64 rows against 6,144 x 2,560 from 79.0 to 59.8 us, against 2,560 x 9,728 from 140.8 to 108.8 (four an SM over
+// more blocks: 100 rows against 2,560 x 4,096 70.4, three 85.0).  Tiles of 72 rows need them, packed: 201 rows against 19,456 x
+// 2,560 565 -> 526.
 // 256 rows against 19,456 x 2,560: 565 us, 45 TFLOP/s (stages of 16 lanes 612; 16 TFLOP/s in 64 x 64 tiles without copies ahead); one chain
 // without packing, 8 x 8 sums a thread or 16 x 16 threads ran at 36 to 46.
 namespace cg = cooperative_groups;
 constexpr int TL_BN = 64, TL_BK = 32, TL_PITCH = TL_BK + 4, TL_STAGES = 2, TL_THREADS = 128;
 
-template <int TMR>
-__global__ __launch_bounds__(TL_THREADS, 4) void sgemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ B,
+template <int TMR, int BLOCKS>
+__global__ __launch_bounds__(TL_THREADS, BLOCKS) void sgemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ B,
                                                                    float* __restrict__ C, int M, int N, int K, long long lda,
                                                                    long long ldb, long long ldc, int seg, int nseg, int m_tiles) {
     constexpr int TL_BM = 8 * TMR, ROWS = TL_BM + TL_BN, STAGE = ROWS * TL_PITCH;
@@ -328,11 +334,16 @@ __global__ __launch_bounds__(TL_THREADS, 4) void sgemm_tile_kernel(const float* 
         if (t < steps) load(t);
         copies_commit();
     }
-    unsigned long long acc[TMR][4];
+    constexpr bool SINGLE = BLOCKS == 3 && TMR <= 8;
+    unsigned long long acc[SINGLE ? 1 : TMR][4];       // packed: the even k in the low half, the odd ones in the high half
+    float even[SINGLE ? TMR : 1][4], odd[SINGLE ? TMR : 1][4];
 #pragma unroll
     for (int i = 0; i < TMR; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < 4; ++j) {
+            if constexpr (SINGLE) even[i][j] = odd[i][j] = 0.f;
+            else acc[i][j] = 0ull;
+        }
     for (int t = 0; t < steps; ++t) {
         copies_wait<TL_STAGES - 2>();
         __syncthreads();
@@ -342,16 +353,30 @@ __global__ __launch_bounds__(TL_THREADS, 4) void sgemm_tile_kernel(const float* 
         const float* b_s = ring + (t % TL_STAGES) * STAGE + (TL_BM + tx) * TL_PITCH;
 #pragma unroll
         for (int k = 0; k < TL_BK; k += 4) {
-            ulonglong2 b[4];
+            if constexpr (SINGLE) {
+                float4 b[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(b_s + 16 * j * TL_PITCH + k);
+                for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(b_s + 16 * j * TL_PITCH + k);
 #pragma unroll
-            for (int i = 0; i < TMR; ++i) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + 8 * i * TL_PITCH + k);
+                for (int i = 0; i < TMR; ++i) {
+                    const float4 a = *reinterpret_cast<const float4*>(a_s + 8 * i * TL_PITCH + k);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) fma2(acc[i][j], a.x, b[j].x);
+                    for (int j = 0; j < 4; ++j) { even[i][j] = fmaf(a.x, b[j].x, even[i][j]); odd[i][j] = fmaf(a.y, b[j].y, odd[i][j]); }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) fma2(acc[i][j], a.y, b[j].y);
+                    for (int j = 0; j < 4; ++j) { even[i][j] = fmaf(a.z, b[j].z, even[i][j]); odd[i][j] = fmaf(a.w, b[j].w, odd[i][j]); }
+                }
+            } else {
+                ulonglong2 b[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(b_s + 16 * j * TL_PITCH + k);
+#pragma unroll
+                for (int i = 0; i < TMR; ++i) {
+                    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + 8 * i * TL_PITCH + k);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) fma2(acc[i][j], a.x, b[j].x);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) fma2(acc[i][j], a.y, b[j].y);
+                }
             }
         }
     }
@@ -360,7 +385,12 @@ __global__ __launch_bounds__(TL_THREADS, 4) void sgemm_tile_kernel(const float* 
 #pragma unroll
     for (int i = 0; i < TMR; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ring[(ty + 8 * i) * SUM_PITCH + tx + 16 * j] = even_plus_odd(acc[i][j]);
+        for (int j = 0; j < 4; ++j) {
+            float v;
+            if constexpr (SINGLE) v = even[i][j] + odd[i][j];
+            else v = even_plus_odd(acc[i][j]);
+            ring[(ty + 8 * i) * SUM_PITCH + tx + 16 * j] = v;
+        }
     if (nseg == 1) {
         __syncthreads();
     } else {
@@ -421,13 +451,13 @@ cudaError_t choose_rows(const float* A, const float* B, float* C, int M, int N, 
     return launch_rows<MT, 3>(A, B, C, M, N, K, lda, ldb, ldc, features, 3 * stage, early, stream);
 }
 
-template <int TMR>
+template <int TMR, int BLOCKS>
 cudaError_t launch_tile(const float* A, const float* B, float* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                         cudaStream_t stream) {
     const int m_tiles = (M + 8 * TMR - 1) / (8 * TMR), nseg = segments(K);
     const long long blocks = (long long)m_tiles * ((N + TL_BN - 1) / TL_BN) * nseg;
     if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
-    return launch_pdl_clusters(sgemm_tile_kernel<TMR>, dim3((unsigned)blocks), dim3(TL_THREADS), 0, stream, (unsigned)nseg, A, B, C, M, N, K,
+    return launch_pdl_clusters(sgemm_tile_kernel<TMR, BLOCKS>, dim3((unsigned)blocks), dim3(TL_THREADS), 0, stream, (unsigned)nseg, A, B, C, M, N, K,
                                lda, ldb, ldc, segment(K), nseg, m_tiles);
 }
 }  // namespace
@@ -454,7 +484,16 @@ VCB_API int vcb_sgemm_tn(const float* A, const float* B, float* C, int M, int N,
             const int p = (M + 8 * t - 1) / (8 * t) * (8 * t);
             if (p < padded) { best = t; padded = p; }
         }
-        auto tile = best == 8 ? launch_tile<8> : best == 7 ? launch_tile<7> : best == 6 ? launch_tile<6> : best == 5 ? launch_tile<5> : launch_tile<4>;
+        // blocks of a tile of 64 features, all segments; where three an SM hold them all, and where there are many rounds of tiles of
+        // 72 rows, whose rate is 1.03 to 1.08 times the others', see above
+        const long long columns = (long long)((N + TL_BN - 1) / TL_BN) * segments(K), sms = num_sms();
+        const int high = (M + 71) / 72;
+        const float rate = best == 8 ? 0.4225f : best == 7 ? 0.4137f : 0.40f;
+        if (high * columns > 12 * sms && (float)(72 * high) / 0.434f < (float)padded / rate) best = 9;
+        const bool resident = padded / (8 * best) * columns <= 3 * sms;
+        auto tile = best == 9 ? launch_tile<9, 3> : best == 8 ? (resident ? launch_tile<8, 3> : launch_tile<8, 4>)
+                    : best == 7 ? (resident ? launch_tile<7, 3> : launch_tile<7, 4>)
+                    : best == 6 ? launch_tile<6, 4> : best == 5 ? launch_tile<5, 4> : launch_tile<4, 4>;
         e = tile(A, B, C, M, N, K, lda, ldb, ldc, stream);
     }
     VCB_CHECK_ARG(e == cudaSuccess, "sgemm_tn: M=%d N=%d K=%d: %s", M, N, K, cudaGetErrorString(e));
