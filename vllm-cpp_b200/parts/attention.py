@@ -79,21 +79,18 @@ class AttentionPlan:
 
     def __init__(self, ctx, nh: int, nkv: int, decode_rows: int = DECODE_ROWS, span_rows: int = SPAN_ROWS,
                  cluster_hd: int | None = None, one_slice: bool = False, max_keys: int = 0,
-                 whole_tokens: bool = False, join: bool = False):
+                 whole_tokens: bool = False):
         """``cluster_hd``: the head size, when the kernel that takes the decoded tokens can merge a token's key slices
         within a cluster of its blocks (then the slices are chosen so that all clusters run at once); else None.
         ``one_slice``: no key slices, whatever the contexts.  ``max_keys`` > 0: no query reads more keys than this
         (a window), so the key ranges are sliced as if no context were longer.  ``whole_tokens``: a block of the kernel that
-        takes the decoded tokens is a token and key slice with all heads, and has an SM to itself.  ``join``: the single tokens
-        may be portions of one token among the others (see singles_join_portions)."""
+        takes the decoded tokens is a token and key slice with all heads, and has an SM to itself."""
         g = nh // nkv
         dev = ctx.device
         # int32 arrays go to the device with the step's own staging buffers where the step has them
         upload = getattr(ctx, "upload", None) or (lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev))
         dec = [i for i, n in enumerate(ctx.host_q_len) if n == 1]
         spans = [i for i, n in enumerate(ctx.host_q_len) if n > 1]
-        if join and singles_join_portions(ctx.host_q_len, ctx.host_ctx_len, nkv, max(1, span_rows // min(g, span_rows))):
-            dec, spans = [], [i for i, n in enumerate(ctx.host_q_len) if n > 0]
         self.n_dec = len(dec)
         self.decode_only = bool(dec) and not spans     # every entry of the step is one decoded token (or empty)
         self.nslices = 1
@@ -174,22 +171,6 @@ def stream_pays(plan: AttentionPlan, nkv: int) -> bool:
                 and (plan.longest is None or plan.longest <= STREAM_MAX_CONTEXT))
 
 
-def singles_join_portions(q_len, ctx_len, nkv: int, tokens_a_unit: int) -> bool:
-    """Whether a step's single tokens run as portions of one token in the prompt kernel's queue.  Its persistent blocks
-    (two an SM) then take them beside the portions' units, longest first, where the decode kernel ahead of it holds the SMs
-    until its longest key range is through, read by a block alone (24 tokens over 200 to 3,000 keys beside 2,024: 52 us).
-    A unit of one token walks its keys as slowly as one of 128 rows, so it pays where the longest single key range is no longer
-    than what every block has to walk anyway.  Only for steps whose lengths the host knows."""
-    singles = [c for n, c in zip(q_len, ctx_len) if n == 1]
-    if not singles or len(singles) == sum(1 for n in q_len if n > 0):
-        return False
-    tiles = sum(-(-c // 64) for c in singles)
-    for n, c in zip(q_len, ctx_len):
-        if n > 1:
-            tiles += sum(-(-(c - n + min(n, q0 + tokens_a_unit)) // 64) for q0 in range(0, n, tokens_a_unit))
-    return -(-max(singles) // 64) * BLOCKS_PER_SM * ops.num_sms() <= tiles * nkv
-
-
 class GQAAttention(Mixer):
     """params: ``hidden_size``, ``num_heads``, ``num_kv_heads``, ``head_dim``, ``eps``
     (of the per-head norms), ``qk_norm`` (bool), ``window`` (0: all keys), ``has_kv``
@@ -266,10 +247,8 @@ class GQAAttention(Mixer):
         dec_rows, span_rows = (MMA_DECODE_ROWS, MMA_SPAN_ROWS) if mma else (DECODE_ROWS, SPAN_ROWS)
         clustered = hd if mma and CLUSTER_MERGE and torch.cuda.is_available() else None
         always_stream = STREAM_DECODE == 2 and mma and ops.attn_stream_supported(x.dtype, hd, cache.pages.shape[3], nh, nkv)
-        tc = mma and TCGEN05_SPANS and ops.attn_tc_supported(x.dtype, hd, cache.pages.shape[3])
-        join = bool(tc and not self.window and not always_stream and not getattr(ctx, "static", False))
-        plan = ctx.plan(("attention", nh, nkv, mma, clustered, always_stream, join),
-                        lambda: AttentionPlan(ctx, nh, nkv, dec_rows, span_rows, clustered, one_slice=always_stream, join=join))
+        plan = ctx.plan(("attention", nh, nkv, mma, clustered, always_stream),
+                        lambda: AttentionPlan(ctx, nh, nkv, dec_rows, span_rows, clustered, one_slice=always_stream))
         common = dict(nh=nh, nkv=nkv, hd=hd, window=self.window, status=ctx.status, table_row=ctx.slots)
         # many single tokens: more (token, KV head) pairs than blocks that are resident at once
         stream = bool(plan.n_dec) and (always_stream or (
@@ -320,7 +299,7 @@ class GQAAttention(Mixer):
                                plan.dec_items, plan.n_dec * S, dec_rows, part_o, part_ml, **common)
                 if S > 1:
                     ops.attn_merge(part_o, part_ml, plan.dec_rows, out, plan.n_dec, nh, hd, S)
-        if plan.n_span_items and tc:
+        if plan.n_span_items and mma and TCGEN05_SPANS and ops.attn_tc_supported(x.dtype, hd, cache.pages.shape[3]):
             ops.attn_tc(q, out, cache.pages, group.block_table, ctx.q_start, ctx.q_len, ctx.ctx_len,
                         plan.span_items, plan.n_span_items, work=plan.span_work, **common)
         elif plan.n_span_items:
