@@ -163,3 +163,20 @@ def test_single_tokens_beside_portions_stay_with_the_decode_kernels(singles, por
                  types.SimpleNamespace(group=0, pages=torch.zeros(1, 2, nkv, 16, hd, dtype=torch.bfloat16)))
     entries = {kind: sorted({int(e) for items in found for e in items[:, 0]}) for kind, found in taken.items()}
     assert entries == {"single": list(range(len(singles))), "portion": list(range(len(singles), len(c.host_q_len)))}
+
+
+def test_slices_of_engines_for_short_requests(monkeypatch):
+    """A captured step's slices are cut to the positions of the engine only where every slice still is at most one key tile, and
+    not at all in the plain kernel and where a block takes all heads: fewer slices there are further from 64 bits."""
+    monkeypatch.setattr(A.ops, "num_sms", lambda: 148)
+
+    def slices(positions, rows, **kw):
+        c = ctx([1, 1], [0, 0], static=True, bound=8192)
+        c.static_positions = positions
+        return A.AttentionPlan(c, 32, 8, rows, A.MMA_SPAN_ROWS, **kw).nslices
+
+    every = slices(40960, A.MMA_DECODE_ROWS)
+    for positions in (1, 64, 65, 100, 128, 300, 400, 8192):
+        assert slices(positions, A.MMA_DECODE_ROWS) == min(every, (positions + 63) // 64)
+        assert slices(positions, A.DECODE_ROWS) == slices(40960, A.DECODE_ROWS)
+        assert slices(positions, A.MMA_DECODE_ROWS, whole_tokens=True) == slices(40960, A.MMA_DECODE_ROWS, whole_tokens=True)

@@ -108,12 +108,14 @@ class AttentionPlan:
                 if max_keys:
                     longest = max_keys if longest is None else min(longest, max_keys)
                 by_pages = MAX_SLICES if longest is None else max(1, longest // per_slice)
-                # No context is longer than the positions that the engine was set up for: one for short requests takes no more
-                # slices than those have 64 keys (two requests of 50 tokens among 64 positions, 4B sizes: 2,364 -> 2,297 us), in the
-                # plain kernel, which a longer key range holds up more, 32 (three of 400: 4,520 us in nine slices, 5,366 in three).
+                # No context is longer than the positions that the engine was set up for: in the tensor-core kernels, which take 64 keys
+                # at a time, one for short requests has no more slices of a KV head's keys than those have tiles (two requests of 50 tokens among 64
+                # positions, 4B sizes: 2,364 -> 2,297 us).  Fewer than that would take results further from 64 bits (100 positions in
+                # one slice 0.3 to 0.4 %, 300 in four 0.1), as fewer slices do in the plain kernel (32 keys a slice: 0.2 to 1.3 %), which
+                # they do not make faster either (one to three tokens over up to 200 keys 20.5 to 22.5 us, 22.6 to 24.6 so).
                 positions = getattr(ctx, "static_positions", None)
-                if positions is not None:
-                    by_pages = min(by_pages, max(1, positions // (32 if decode_rows == DECODE_ROWS else 64)))
+                if positions is not None and decode_rows != DECODE_ROWS and not whole_tokens:
+                    by_pages = min(by_pages, -(-positions // 64))
             else:
                 longest = self.longest = max(ctx.host_ctx_len[i] for i in dec)
                 if max_keys:
