@@ -89,3 +89,23 @@ def test_portions_whose_launches_hide_run_kernel_by_kernel():
     model = types.SimpleNamespace(layers=[layer], order=[types.SimpleNamespace(layer=0)] * 36)
     assert 30 < _launches_hide_from(model) < 60
     assert _launches_hide_from(types.SimpleNamespace()) is None
+
+
+def test_portions_that_fill_their_bucket_stay_captured_beyond_the_limit():
+    """Beyond the limit a 32-bit engine's portions run kernel by kernel only where their bucket has more rows of products, in whole
+    tiles of 32 to 64 rows, than would make up for the launches."""
+    r = fake_runner()
+    r.capture_limit = 44
+    sizes = {n: r.portion_size([entry(n)]) for n in range(2, 513)}
+    for low, high, padded in ((2, 44, (16, 32, 64)), (57, 64, (64,)), (81, 96, (96,)), (121, 128, (128,)), (169, 192, (192,)), (241, 256, (256,)),
+                              (361, 384, (384,)), (505, 512, (512,))):
+        assert all(sizes[n] in padded for n in range(low, high + 1)), (low, high)
+    for low, high in ((45, 56), (65, 80), (97, 120), (129, 168), (193, 240), (257, 320), (385, 448)):
+        assert all(sizes[n] is None for n in range(low, high + 1)), (low, high)
+    singles = [entry(1, slot=i) for i in range(8)]
+    assert r.mixed_size(singles + [entry(56, slot=9)]) == (8, 64) and r.mixed_size(singles + [entry(88, slot=9)]) == (8, 96)
+    assert r.mixed_size(singles + [entry(40, slot=9)]) is None
+    r.capture_limit = 23
+    assert [r.portion_size([entry(n)]) for n in (24, 28, 32, 33, 40, 64)] == [32, 32, 32, None, None, 64]
+    r.capture_limit = None
+    assert all(r.portion_size([entry(n)]) is not None for n in range(2, 513))

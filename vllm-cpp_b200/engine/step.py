@@ -181,13 +181,28 @@ class StepContext:
 
 def _launches_hide_from(model) -> int | None:
     """Tokens beyond which the 32-bit products of a portion take the GPU half as long again as the host needs to launch a layer:
-    some 150 us a run of the execution order, against 40 TFLOP/s.  Experts, of which a token meets a few, do not count."""
+    some 150 us a run of the execution order, against 40 TFLOP/s.  Routed feed-forward parts, whose kernels cost the host more too, are left
+    out whole, a shared expert among them: with them the number is larger, and more portions stay captured."""
     weights = 0
     for run in getattr(model, "order", ()):
         for part in model.layers[run.layer].parts.values():
             if not hasattr(part, "top"):
                 weights += sum(s.shape[0] * s.shape[1] for s in part.tensor_specs() if s.role == "matrix" and len(s.shape) == 2 and min(s.shape) > 0)
     return max(1, int(1.5 * 150e-6 * 40e12 * len(model.order) / (2 * weights))) if weights else None
+
+
+def _padding_pays(limit: int | None, tokens: int, padded: int) -> bool:
+    """Whether a portion of ``tokens`` (single tokens beside it counted) runs as the captured step of ``padded`` token rows.  ``limit``:
+    see _launches_hide_from; up to it, and without one, always.  Beyond it launches that nothing hides cost a layer 5 to 17 us for a
+    portion alone and up to 39 beside single tokens, and ``limit`` rows of products 225: so not where padding adds a sixth of ``limit`` rows
+    or more.  Rows as the products have them, in the tiles of 32 to 64 that pad them least (sgemm.cu).  4B sizes, limit 44, captured and kernel by
+    kernel in ms, waited for after each: 45 tokens 17.0 and 15.8, 56 17.3 and 16.6, 60 17.0 and 17.6, 64 17.3 and 17.9, 80 23.8 and 21.3, 96
+    24.0 and 24.2, 201 54.1 and 47.9, 256 54.5 and 55.0; beside eight single tokens 40 18.6 and 17.9, 44 18.3 and 18.3, 56 18.6 and 19.9.  8B sizes, limit
+    23: 24 tokens 17.3 and 17.5, 40 28.0 and 20.2; 28 layers of 1,024 lanes, limit 286: 287 tokens 14.8 and 13.5, 384 15.4 and 15.6."""
+    if limit is None or tokens <= limit:
+        return True
+    rows, padded_rows = (min(-(-n // tile) * tile for tile in range(32, 65, 8)) for n in (tokens, padded))
+    return 6 * (padded_rows - rows) < limit
 
 
 class ModelRunner:
@@ -243,7 +258,7 @@ class ModelRunner:
             self.size_workspace(max_step_tokens)
         # A captured step pads a portion to its bucket, which hides the host's launches.  32-bit products are bound by
         # multiply-adds: there a portion that takes the GPU longer than its launches take the host runs kernel by kernel over
-        # its own tokens (201 tokens of the 4B sizes: 51.7 ms padded to 256 and replayed, 48.8 so).
+        # its own tokens, where its bucket has more rows of products than that saves (see _padding_pays).
         self.capture_limit = _launches_hide_from(model) if dtype == torch.float32 and self.cuda_graphs else None
         self.graph_replays = 0
         self.launches_per_graph: dict[tuple, int] = {}
@@ -360,22 +375,23 @@ class ModelRunner:
     def portion_size(self, entries) -> int | None:
         """The padded token count of the captured step that would run these entries: one entry, a prompt portion of
         up to 512 tokens, logits wanted at most at its last token.  Kernel by kernel the host needs some twenty
-        microseconds a launch, which for a short portion is twice the time the GPU needs."""
+        microseconds a launch, which for a short portion is twice the time the GPU needs.  32-bit portions beyond
+        ``capture_limit`` are captured only where padding adds next to no rows (see _padding_pays)."""
         if not self.cuda_graphs or len(entries) != 1:
             return None
         e = entries[0]
         n = len(e.tokens)
         if n < 2 or n > self.PORTION_BUCKETS[-1] or e.want not in ([], [n - 1]):
             return None
-        if n > (getattr(self, "capture_limit", None) or n):
-            return None
-        return next(b for b in self.PORTION_BUCKETS if b >= n)
+        padded = next(b for b in self.PORTION_BUCKETS if b >= n)
+        return padded if _padding_pays(getattr(self, "capture_limit", None), n, padded) else None
 
     def mixed_size(self, entries) -> tuple[int, int] | None:
         """(single-token slots, token rows) of the captured step that would run these entries: single-token
         entries first, then one to four prompt portions of two tokens or more with logits wanted at their last
         token or nowhere, up to 64 single tokens and 256 tokens in all (beyond that the GPU needs longer for a step
-        than the host needs to launch it kernel by kernel).  None: they run kernel by kernel."""
+        than the host needs to launch it kernel by kernel).  Beyond ``capture_limit`` as for a lone portion.  None: they run
+        kernel by kernel."""
         if not self.cuda_graphs or len(entries) < 2:
             return None
         n_single = 0
@@ -390,11 +406,11 @@ class ModelRunner:
             if n < 2 or e.want not in ([], [n - 1]):
                 return None
             tokens += n
-        if n_single + tokens > (getattr(self, "capture_limit", None) or n_single + tokens):
-            return None
         singles = next(b for b in self.MIXED_SINGLES if b >= n_single)
         rows = next((b for b in self.MIXED_TOKENS if b >= singles + tokens), None)
-        return None if rows is None else (singles, rows)
+        if rows is None or not _padding_pays(getattr(self, "capture_limit", None), n_single + tokens, rows):
+            return None
+        return singles, rows
 
     def _mixed_updates(self, singles: int, rows: int) -> int:
         """Block-table entries that a captured mixed step's buffer has room for."""
