@@ -151,15 +151,15 @@ __device__ __forceinline__ float gemm_act(float x, int act) {
 
 // MT = 128-feature tiles per work unit that share one token tile (2 halves the bytes that cross L2 per flop);
 // ACC = accumulator buffers in TMEM (2: the epilogue of one unit overlaps the MMAs of the next).
-template <int BN, int STAGES, int MT, int ACC>
+template <int BN, int STAGES, int MT, int ACC, bool FEWER>
 struct Smem {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = MT * A_BYTES + B_BYTES;
-    // Up to 128 tokens a unit may have fewer features than a tile has lanes (GemmArgs::unit_rows): its stages are shorter, and
-    // there are as many more of them as fit into the same room.
-    static constexpr bool FLEX = MT == 1 && BN <= 128;
-    static constexpr int MAX_STAGES = FLEX ? 16 : STAGES;
+    // FEWER (up to 128 tokens): a unit has fewer features than a tile has lanes (GemmArgs::unit_rows), its stages are shorter, and
+    // there are as many more of them as fit into the same room.  A kernel of its own: with the stages' number and size no constants
+    // where units have 128 features either, captured steps of 9 to 32 tokens took a percent longer (4B sizes, 16 tokens 2,879 -> 2,909 us).
+    static constexpr int MAX_STAGES = FEWER ? 16 : STAGES;
     static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
     static constexpr int NUM_BARS = 2 * MAX_STAGES + 2 * ACC;
     // a stage's 128 rows are read whole by the products, whatever lies beyond the unit's features: the last stage leaves room for that
@@ -277,6 +277,21 @@ __device__ __forceinline__ void xielu_store(const uint32_t (&v)[CHUNK / 16][16],
 template <int CHUNK>
 __device__ __forceinline__ void plain_store(const uint32_t (&v)[CHUNK / 16][16], void* out, int out_dtype, size_t at, long long ldc, int m, int M,
                                             int t0, int N, int lane, int act) {
+    // (the sums as they are have a path of their own, ahead of all else: through the values' second copy below a captured step of 16 tokens of
+    // the 4B sizes took 2,875 us, so 2,850)
+    if (act == 0 && out_dtype == VCB_F32) {
+        if (m >= M) return;
+        float* o = reinterpret_cast<float*>(out) + at + (size_t)t0 * ldc + m;
+        if (t0 + CHUNK <= N) {
+#pragma unroll
+            for (int jj = 0; jj < CHUNK; ++jj) o[(size_t)jj * ldc] = __uint_as_float(v[jj / 16][jj % 16]);
+        } else {
+#pragma unroll
+            for (int jj = 0; jj < CHUNK; ++jj)
+                if (t0 + jj < N) o[(size_t)jj * ldc] = __uint_as_float(v[jj / 16][jj % 16]);
+        }
+        return;
+    }
     float r[CHUNK];
 #pragma unroll
     for (int jj = 0; jj < CHUNK; ++jj) r[jj] = __uint_as_float(v[jj / 16][jj % 16]);
@@ -410,11 +425,11 @@ __device__ __forceinline__ void tile_of(int idx, int m_tiles, int n_tiles, int& 
 // Persistent: each block walks the work units blockIdx.x, blockIdx.x + gridDim.x, ...; a unit is
 // (feature tile group, token tile, k-slice).  The stage ring and the accumulator ring run on across units, so
 // the loads of the next unit are in flight while the current one is multiplied and the one before is stored.
-template <int BN, int STAGES, int MT, int ACC>
+template <int BN, int STAGES, int MT, int ACC, bool FEWER>
 __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                     const __grid_constant__ CUtensorMap map_x,
                                                                     GemmArgs g) {
-    using L = Smem<BN, STAGES, MT, ACC>;
+    using L = Smem<BN, STAGES, MT, ACC, FEWER>;
     constexpr uint32_t ACC_COLS = BN < 32 ? 32 : BN;            // columns of one 128-feature accumulator
     constexpr int CHUNK = BN % 64 == 0 ? 64 : (BN % 32 == 0 ? 32 : 16);   // accumulator columns read per wait in the epilogue
     constexpr uint32_t USED_COLS = ACC * MT * ACC_COLS;
@@ -435,9 +450,9 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
     tl_mark(VCB_TL_GEMM, 0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_kb = (g.K + BK - 1) / BK;
-    const int unit_rows = L::FLEX ? g.unit_rows : BM * MT;   // rows of W per unit
-    const int stages = L::FLEX ? g.stages : STAGES;
-    const int a_bytes = L::FLEX ? unit_rows * BK * 2 : MT * L::A_BYTES;
+    const int unit_rows = FEWER ? g.unit_rows : BM * MT;   // rows of W per unit
+    const int stages = FEWER ? g.stages : STAGES;
+    const int a_bytes = FEWER ? unit_rows * BK * 2 : MT * L::A_BYTES;
     const int stage_bytes = a_bytes + L::B_BYTES;
     const int m_tiles = (g.M + unit_rows - 1) / unit_rows;
     const int n_tiles = (g.N + BN - 1) / BN;
@@ -610,11 +625,11 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
             tc_fence_after();
             const uint32_t tmem_d = tmem_base + a * (MT * ACC_COLS);
             const size_t zoff = (size_t)z * g.split_stride;
-            const int m_end = L::FLEX ? min(g.M, m0 + unit_rows) : g.M;     // lanes beyond a unit's features hold what lay behind them in the ring
+            const int m_end = FEWER ? min(g.M, m0 + unit_rows) : g.M;     // lanes beyond a unit's features hold what lay behind them in the ring
 #pragma unroll 1
             for (int cc = 0; cc < MT * BN; cc += CHUNK) {
                 const int mt = cc / BN, c0 = cc % BN;
-                if (n0 + c0 >= g.N || (L::FLEX && m0 + q * 32 >= m_end && g.qe.q_out == nullptr)) continue;   // uniform over the warp
+                if (n0 + c0 >= g.N || (FEWER && m0 + q * 32 >= m_end)) continue;   // uniform over the warp
                 const int m = m0 + mt * BM + q * 32 + lane;
                 // several TMEM loads in flight before one wait: their latencies overlap
                 uint32_t v[CHUNK / 16][16];
@@ -622,7 +637,7 @@ __global__ __launch_bounds__(NTHREADS, 1) void gemm_bf16_tn_kernel(const __grid_
                 for (int b = 0; b < CHUNK / 16; ++b)
                     tc_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * ACC_COLS + c0 + 16 * b), v[b]);
                 tc_wait_ld();
-                if constexpr (L::EPI_BYTES > 0) {
+                if constexpr (L::EPI_BYTES > 0 && !FEWER) {
                     if (g.qe.q_out != nullptr) {     // uniform over the block: every warp takes part in the barriers
                         float* stage = reinterpret_cast<float*>(gen + L::EPI_OFFSET);
 #pragma unroll
@@ -1027,21 +1042,12 @@ int choose_unit_rows(int M, int n_tiles, int splits, int kb_per_split) {
     return BM;
 }
 
-template <int BN, int STAGES, int MT, int ACC>
-int launch_maps(const void* W, long long w_rows, const void* X, GemmArgs g, long long ldw, long long ldx, int splits,
-                cudaStream_t stream) {
-    using L = Smem<BN, STAGES, MT, ACC>;
-    if (!L::FLEX) {
-        g.unit_rows = BM * MT;
-    } else {
-        // (a tile of a grouped product and a head of the q, k, v epilogue are 128 features)
-        if (g.tile_group != nullptr || g.qe.q_out != nullptr) g.unit_rows = BM;
-        else if (g.unit_rows == 0) g.unit_rows = choose_unit_rows(g.M, (g.N + BN - 1) / BN, splits, g.kb_per_split);
-        g.stages = L::stages(g.unit_rows);
-    }
+template <int BN, int STAGES, int MT, int ACC, bool FEWER>
+int launch_units(const void* W, long long w_rows, const void* X, const GemmArgs& g, long long ldw, long long ldx, int splits, cudaStream_t stream) {
+    using L = Smem<BN, STAGES, MT, ACC, FEWER>;
     CUtensorMap mw, mx;
-    if (!tensor_map(W, w_rows, g.K, ldw, L::FLEX ? g.unit_rows : BM, &mw) || !tensor_map(X, g.N, g.K, ldx, BN, &mx)) return -3;
-    auto kern = gemm_bf16_tn_kernel<BN, STAGES, MT, ACC>;
+    if (!tensor_map(W, w_rows, g.K, ldw, FEWER ? g.unit_rows : BM, &mw) || !tensor_map(X, g.N, g.K, ldx, BN, &mx)) return -3;
+    auto kern = gemm_bf16_tn_kernel<BN, STAGES, MT, ACC, FEWER>;
     static bool opted = false;
     if (!opted) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
@@ -1056,6 +1062,22 @@ int launch_maps(const void* W, long long w_rows, const void* X, GemmArgs g, long
     launch_pdl(kern, dim3(grid), dim3(NTHREADS), L::TOTAL, stream, mw, mx, g);
     VCB_CHECK_LAUNCH("gemm_bf16_tn");
     return 0;
+}
+
+template <int BN, int STAGES, int MT, int ACC>
+int launch_maps(const void* W, long long w_rows, const void* X, GemmArgs g, long long ldw, long long ldx, int splits, cudaStream_t stream) {
+    if constexpr (MT == 1 && BN <= 128) {
+        // (a tile of a grouped product and a head of the q, k, v epilogue are 128 features)
+        if (g.tile_group != nullptr || g.qe.q_out != nullptr) g.unit_rows = BM;
+        else if (g.unit_rows == 0) g.unit_rows = choose_unit_rows(g.M, (g.N + BN - 1) / BN, splits, g.kb_per_split);
+        if (g.unit_rows < BM) {
+            g.stages = Smem<BN, STAGES, MT, ACC, true>::stages(g.unit_rows);
+            return launch_units<BN, STAGES, MT, ACC, true>(W, w_rows, X, g, ldw, ldx, splits, stream);
+        }
+    } else {
+        g.unit_rows = BM * MT;
+    }
+    return launch_units<BN, STAGES, MT, ACC, false>(W, w_rows, X, g, ldw, ldx, splits, stream);
 }
 
 template <int BN, int STAGES, int MT, int ACC>
