@@ -396,8 +396,9 @@ __global__ __launch_bounds__(NTHREADS + (KIND != ROWS_PLAIN ? 32 * KEY_WARPS : 0
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // What no kernel of the step writes -- the work items, the entries' lengths, the block tables -- is read before the wait:
-    // the block's first unit, and the first page of its keys (each a round trip to memory behind another).
+    // What is in place before the step's first model kernel starts is read before the wait: the block's first unit, and the first page
+    // of its keys (each a round trip to memory behind another).  Work items and lengths are copied, an ordinary stream operation; the
+    // block tables are written by scatter_i32_kernel, which holds its early launch back for this (a trigger there would break it).
     Unit u;
     bool has = read_unit<OPT>(a, (int)blockIdx.x, u);
     const int pages_per_tile = BNK / ps;

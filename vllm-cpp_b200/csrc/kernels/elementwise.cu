@@ -717,11 +717,15 @@ __global__ void scatter_i32_kernel(int* __restrict__ dst, const int* __restrict_
                                    const int* __restrict__ count, int capacity, long long dst_size) {
     // No early trigger here: the kernel after this one then starts only when this one has ended, and every later
     // kernel of the step after that, so all of them may read the block tables before their own dependency wait
-    // (the attention kernel asks for old key tiles that early).
+    // (the attention kernels ask for their units and for old key tiles that early).  Only a wait makes what a kernel wrote visible
+    // by itself, so the entries are fenced: whoever starts after the last block has left finds them.
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = min(*count, capacity);
-    if (i < n && idx[i] >= 0 && idx[i] < dst_size) dst[idx[i]] = val[i];
+    if (i < n && idx[i] >= 0 && idx[i] < dst_size) {
+        dst[idx[i]] = val[i];
+        __threadfence();
+    }
 }
 
 // count lives on the device so that a captured launch can serve any number of updates up to capacity
