@@ -196,6 +196,9 @@ __global__ __launch_bounds__(1024) void sample_kernel(const float* __restrict__ 
 // predicated sums and a comparison of places were most), so a score that reaches no threshold is left at one comparison of floats.
 // 64 rows of 151,936 with penalty, temperature and nucleus: 1,620 us with a block a row, 56 here (71 with keys and sums for every
 // score); with a temperature alone 41 (56 with two logarithms for every score near the maximum).
+// Scores like noise, most of which reach thresholds, lose where a block has an SM to itself (a few rows, or more than 192,000 scores: one
+// row of 151,936 62 -> 64 us, of 262,144 91 -> 98) and gain elsewhere (32 rows of 151,936 123 -> 112); a model's gain in both (one row 20.5 -> 18.7, of
+// 262,144 28.0 -> 24.5).  Sums under predicates instead of branches take back half of either.
 namespace cg = cooperative_groups;
 constexpr size_t CLUSTER_MAX_SMEM = 192 * 1024;      // beside ClusterShared (18 KB)
 constexpr int CL_THREADS = 512, CL_WARPS = CL_THREADS / 32, CL_BLOCKS = 8, NT = 7, CAND = 1024;
@@ -522,6 +525,11 @@ __global__ __launch_bounds__(CL_THREADS, 2) void sample_cluster_kernel(const flo
 // Two-stage variant for rows that need no nucleus cut (top_p >= 1 or greedy): the vocabulary is dealt to
 // `nb` blocks per row, each leaves its best (value, index), and the last stage picks among them with the same
 // lowest-index rule, so the token equals the single-block kernel's.
+// BOUNDED: may_draw before the logarithms.  A thread's best draw has to rise before that spares any: with 28 to 43 scores a thread it
+// costs 5 to 10 % more (31 rows of 190,000 37 us without it, 41 with; 100 of 32,000 32 and 36), at 57 to 64 a percent less (128 of 65,536
+// 58.7 and 58.1), from 128 on it saves 12 to 15 % (64 of 262,144 129 and 112, 128 of 262,144 237 and 203).
+constexpr int BOUNDED_FROM = 56;
+template <bool BOUNDED>
 __global__ __launch_bounds__(512) void sample_part_kernel(const float* __restrict__ logits, long long row_stride, int V,
                                                           const RowParams* __restrict__ params,
                                                           const int* __restrict__ counts_table, float* __restrict__ part_v,
@@ -546,7 +554,7 @@ __global__ __launch_bounds__(512) void sample_part_kernel(const float* __restric
         if (!greedy) {
             if (s + GUMBEL_MAX < best) continue;
             const float u = uniform01(key, (unsigned int)i);
-            if (!may_draw(s, u, best)) continue;
+            if (BOUNDED && !may_draw(s, u, best)) continue;
             s -= logf(-logf(u));
         }
         if (s > best || (s == best && i < best_i)) { best = s; best_i = i; }
@@ -628,8 +636,8 @@ VCB_API int vcb_sample_split(const float* logits, long long row_stride, int n_ro
                              cudaStream_t stream) {
     if (n_rows == 0) return 0;
     VCB_CHECK_ARG(n_rows > 0 && V > 0 && row_stride >= V && nb >= 1 && nb <= 1024, "sample_split: bad sizes");
-    launch_pdl(sample_part_kernel, dim3(n_rows, nb), dim3(512), 0, stream, logits, row_stride, V, (const RowParams*)params,
-               counts_table, part_v, part_i);
+    auto part = (V + nb - 1) / nb > BOUNDED_FROM * 512 ? sample_part_kernel<true> : sample_part_kernel<false>;
+    launch_pdl(part, dim3(n_rows, nb), dim3(512), 0, stream, logits, row_stride, V, (const RowParams*)params, counts_table, part_v, part_i);
     VCB_CHECK_LAUNCH("sample_part");
     launch_pdl(sample_pick_kernel, dim3(n_rows), dim3(32), 0, stream, part_v, part_i, nb, out);
     VCB_CHECK_LAUNCH("sample_pick");
