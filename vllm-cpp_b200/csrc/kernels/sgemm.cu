@@ -290,7 +290,7 @@ __global__ __launch_bounds__(32 * SEGMENTS, 2) void sgemm_rows_kernel(const floa
 // memory, rows padded by 16 bytes (eight features: eight different groups of four banks), two stages of 32 lanes of K.
 // Four blocks an SM, or three (BLOCKS), whose threads then have 168 registers instead of 128.  What bounds it is the multiply-add
 // pipe, kept waiting by operands in the same register banks.  Over many rounds of blocks four an SM are the better ones, but in 128
-// registers tiles of 56 and 64 rows spill, and where all blocks are resident at once that is not hidden: three an SM with single
+// registers tiles of 56 and 64 rows spill, and where all blocks are resident at once that is not hidden: two to three an SM with single
 // multiply-adds take 64 rows against 6,144 x 2,560 from 79.0 to 59.8 us, against 2,560 x 9,728 from 140.8 to 108.8 (four an SM over
 // more blocks: 100 rows against 2,560 x 4,096 70.4, three 85.0).  Tiles of 72 rows need them, packed: 201 rows against 19,456 x
 // 2,560 565 -> 526.
@@ -484,13 +484,16 @@ VCB_API int vcb_sgemm_tn(const float* A, const float* B, float* C, int M, int N,
             const int p = (M + 8 * t - 1) / (8 * t) * (8 * t);
             if (p < padded) { best = t; padded = p; }
         }
-        // blocks of a tile of 64 features, all segments; where three an SM hold them all, and where there are many rounds of tiles of
-        // 72 rows, whose rate is 1.03 to 1.08 times the others', see above
-        const long long columns = (long long)((N + TL_BN - 1) / TL_BN) * segments(K), sms = num_sms();
-        const int high = (M + 71) / 72;
-        const float rate = best == 8 ? 0.4225f : best == 7 ? 0.4137f : 0.40f;
-        if (high * columns > 12 * sms && (float)(72 * high) / 0.434f < (float)padded / rate) best = 9;
-        const bool resident = padded / (8 * best) * columns <= 3 * sms;
+        // blocks of a tile of 64 features, all segments; see above for three blocks an SM and tiles of 72 rows.  Against four blocks an SM and no
+        // tiles of 72 rows, over 560 products (18 matrices of 256 to 12,288 lanes, 17 to 2,048 rows, weights from HBM) this rule is 2 % faster on
+        // average and nowhere more than 1.3 % slower.  Three wherever they hold all blocks lost up to 22 % with less than two an SM (100 rows against
+        // 3,072 x 1,024 34 -> 42 us: alone on its way a block waits for its own multiply-adds, and packed ones are half as many; clusters of
+        // two segments lose up to there, the others up to one an SM), tiles of 72 rows up to 9 % where others pad as little (400 rows against
+        // 2,560 x 9,728 517 -> 565).
+        const int nseg = segments(K), high = (M + 71) / 72;
+        const long long columns = (long long)((N + TL_BN - 1) / TL_BN) * nseg, sms = num_sms(), blocks = padded / (8 * best) * columns;
+        if (high * columns > 12 * sms && (72ll * high * 100 <= 97ll * padded || (72ll * high <= padded && nseg <= 4))) best = 9;
+        const bool resident = blocks <= 3 * sms && (2 * blocks <= sms || blocks > (nseg == 2 ? 2 : 1) * sms);
         auto tile = best == 9 ? launch_tile<9, 3> : best == 8 ? (resident ? launch_tile<8, 3> : launch_tile<8, 4>)
                     : best == 7 ? (resident ? launch_tile<7, 3> : launch_tile<7, 4>)
                     : best == 6 ? launch_tile<6, 4> : best == 5 ? launch_tile<5, 4> : launch_tile<4, 4>;
