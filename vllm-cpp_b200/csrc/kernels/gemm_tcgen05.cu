@@ -1209,38 +1209,40 @@ int launch_shape(int shape, const void* W, const void* X, GemmArgs g, long long 
 // sizes (1,024 to 34,816 features, 130 to 4,096 tokens, K of 256 to 9,728), the others at 3,686 (heads 1,440).  Taken by the
 // estimate the products are on average 0.5 % (plain), 0.3 (SiLU-gate), 0.4 (k-slices), 0.3 (xIELU) and 1.0 (heads) from the best
 // shape; by numbers fitted to single launches and to the epilogues before they shared columns between lanes, 3.9 %, 1.3 and 4.0, and up
-// to 48 (1,024 features of 256 lanes, 911 tokens).
-enum Epilogue { EPI_PLAIN = 0, EPI_PARTIAL, EPI_GATE, EPI_XIELU, EPI_HEADS, EPI_COUNT };
+// to 48 (1,024 features of 256 lanes, 911 tokens).  32-bit sums without k-slices (EPI_SUMS: twice the bytes to store) are fitted to half of 631
+// sizes and 0.8 % from the best shape on the other half; by the plain numbers 1.3, and up to 15 on 512 lanes (10,240 features, 2,048 tokens 26.2 ->
+// 30.1 us).
+enum Epilogue { EPI_PLAIN = 0, EPI_PARTIAL, EPI_GATE, EPI_XIELU, EPI_HEADS, EPI_SUMS, EPI_COUNT };
 struct UnitTime { float k_block, busy, start, drain, once, ragged; };      // k_block 0: not taken
 struct UnitShape { int shape, tiles, tokens, blocks, chunk; UnitTime time[EPI_COUNT]; };
 const UnitShape UNIT_SHAPES[] = {
     {SHAPE_PAIR, 2, 256, 2, 64,
      {{0.264f, 0.28f, 1.5f, 0.4f, 4.6f, 0.2f}, {0.255f, 0.38f, 1.3f, 3.0f, 2.5f, 0.1f}, {0.276f, 0.28f, 0.9f, 3.3f, 1.6f, 0.1f},
-      {0.280f, 0.24f, 2.3f, 4.0f, 7.8f, 0.0f}, {0.254f, 0.16f, 8.6f, 8.6f, 11.4f, 0.0f}}},
+      {0.280f, 0.24f, 2.3f, 4.0f, 7.8f, 0.0f}, {0.254f, 0.16f, 8.6f, 8.6f, 11.4f, 0.0f}, {0.260f, 0.34f, 2.0f, 0.9f, 3.4f, 0.1f}}},
     {SHAPE_PAIR_TOKENS + 224, 2, 224, 2, 32,
      {{0.268f, 0.21f, 1.3f, 3.0f, 1.7f, 0.0f}, {0.248f, 0.33f, 1.3f, 0.0f, 5.0f, 0.3f}, {0.274f, 0.22f, 0.9f, 3.5f, 1.4f, 0.1f},
-      {0.277f, 0.20f, 2.5f, 4.2f, 6.8f, 0.0f}, {0.258f, 0.07f, 8.5f, 4.5f, 13.2f, 0.0f}}},
+      {0.277f, 0.20f, 2.5f, 4.2f, 6.8f, 0.0f}, {0.258f, 0.07f, 8.5f, 4.5f, 13.2f, 0.0f}, {0.262f, 0.29f, 1.6f, 2.7f, 1.1f, 0.2f}}},
     {SHAPE_PAIR_TOKENS + 192, 2, 192, 2, 64,
      {{0.268f, 0.16f, 1.0f, 1.9f, 2.9f, 0.4f}, {0.264f, 0.19f, 0.8f, 2.4f, 3.1f, 0.4f}, {0.278f, 0.16f, 0.7f, 2.6f, 2.1f, 0.3f},
-      {0.284f, 0.14f, 1.8f, 3.0f, 8.5f, 0.4f}, {0.283f, 0.00f, 6.2f, 9.2f, 8.5f, 0.0f}}},
+      {0.284f, 0.14f, 1.8f, 3.0f, 8.5f, 0.4f}, {0.283f, 0.00f, 6.2f, 9.2f, 8.5f, 0.0f}, {0.270f, 0.20f, 1.3f, 2.2f, 1.8f, 0.4f}}},
     {SHAPE_PAIR_TOKENS + 160, 2, 160, 2, 32,
      {{0.280f, 0.11f, 0.8f, 2.3f, 2.4f, 0.1f}, {0.264f, 0.18f, 0.6f, 2.2f, 3.0f, 0.2f}, {0.282f, 0.11f, 0.6f, 2.7f, 2.0f, 0.2f},
-      {0.284f, 0.14f, 1.5f, 3.2f, 7.7f, 0.0f}, {0.274f, 0.00f, 5.5f, 3.1f, 13.7f, 0.0f}}},
+      {0.284f, 0.14f, 1.5f, 3.2f, 7.7f, 0.0f}, {0.274f, 0.00f, 5.5f, 3.1f, 13.7f, 0.0f}, {0.277f, 0.14f, 1.0f, 2.0f, 2.0f, 0.2f}}},
     {SHAPE_N256, 1, 256, 1, 64,
      {{0.309f, 0.26f, 0.9f, 3.0f, 0.8f, 0.1f}, {0.296f, 0.37f, 1.7f, 3.0f, 0.6f, 0.0f}, {0.315f, 0.26f, 0.5f, 3.4f, 0.4f, 0.2f},
-      {0.349f, 0.14f, 2.3f, 4.3f, 5.8f, 0.0f}, {0.322f, 0.05f, 8.0f, 7.7f, 10.7f, 0.0f}}},
+      {0.349f, 0.14f, 2.3f, 4.3f, 5.8f, 0.0f}, {0.322f, 0.05f, 8.0f, 7.7f, 10.7f, 0.0f}, {0.294f, 0.35f, 2.0f, 3.0f, 0.0f, 0.1f}}},
     {SHAPE_N128, 1, 128, 1, 64,
      {{0.240f, 0.14f, 0.7f, 1.5f, 2.5f, 0.2f}, {0.237f, 0.18f, 0.7f, 2.0f, 2.2f, 0.2f}, {0.247f, 0.13f, 0.4f, 2.0f, 1.6f, 0.2f},
-      {0.254f, 0.16f, 1.1f, 2.6f, 7.1f, 0.0f}, {0.261f, 0.00f, 3.5f, 6.7f, 7.4f, 0.0f}}},
+      {0.254f, 0.16f, 1.1f, 2.6f, 7.1f, 0.0f}, {0.261f, 0.00f, 3.5f, 6.7f, 7.4f, 0.0f}, {0.241f, 0.13f, 0.9f, 1.7f, 1.3f, 0.3f}}},
     {SHAPE_M256_N256, 2, 256, 1, 64,
      {{0.543f, 0.26f, 0.0f, 4.5f, 2.8f, 0.3f}, {}, {0.537f, 0.30f, 0.0f, 5.6f, 2.7f, 0.2f},
-      {0.563f, 0.32f, 0.0f, 7.7f, 8.4f, 0.0f}, {}}},
+      {0.563f, 0.32f, 0.0f, 7.7f, 8.4f, 0.0f}, {}, {0.537f, 0.32f, 0.0f, 5.2f, 2.2f, 0.1f}}},
     {SHAPE_M256_N192, 2, 192, 1, 64,
      {{0.453f, 0.24f, 0.0f, 3.2f, 2.8f, 0.6f}, {}, {0.435f, 0.31f, 0.0f, 3.9f, 2.6f, 0.6f},
-      {0.493f, 0.21f, 0.0f, 5.8f, 8.6f, 0.9f}, {}}},
+      {0.493f, 0.21f, 0.0f, 5.8f, 8.6f, 0.9f}, {}, {0.454f, 0.28f, 0.0f, 4.1f, 1.7f, 0.6f}}},
     {SHAPE_M256_N160, 2, 160, 1, 32,
      {{0.410f, 0.23f, 0.0f, 3.1f, 2.6f, 0.3f}, {}, {0.390f, 0.33f, 0.0f, 3.9f, 2.6f, 0.3f},
-      {0.457f, 0.19f, 0.0f, 5.3f, 8.4f, 0.4f}, {}}},
+      {0.457f, 0.19f, 0.0f, 5.3f, 8.4f, 0.4f}, {}, {0.412f, 0.26f, 0.0f, 3.3f, 2.0f, 0.1f}}},
 };
 
 // For M features, N tokens, inner size K.
@@ -1289,7 +1291,7 @@ VCB_API int vcb_gemm_bf16_tn_shape(const void* W, const void* X, void* out, int 
     splits = (total_kb + kb_per_split - 1) / kb_per_split;
     GemmArgs g{out, out_dtype, M, N, K, ldc, split_stride, kb_per_split, splits, 0, status};
     if ((flags & VCB_GEMM_AFTER_SMALL_KERNEL) && N <= 16 && vcb_pdl_enabled()) pf_settings(&g.pf_tiles, &g.pf_delay_ns);
-    return launch_shape(shape < 0 ? choose_shape(M, N, K, splits, splits > 1 ? EPI_PARTIAL : EPI_PLAIN) : shape, W, X, g, ldw, ldx, splits, stream);
+    return launch_shape(shape < 0 ? choose_shape(M, N, K, splits, splits > 1 ? EPI_PARTIAL : out_dtype == VCB_F32 ? EPI_SUMS : EPI_PLAIN) : shape, W, X, g, ldw, ldx, splits, stream);
 }
 
 // out[t][m] = xIELU(W[m] . X[t]), bfloat16, the activation in the epilogue: what bias_act does with the sums of a product
